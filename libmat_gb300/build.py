@@ -24,6 +24,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
               "-Xptxas", "-O3", "-I" + os.path.join(ROOT, "include")]
 CUDA_UNITS = {
     "rpd_clip.cu": ["-fmad=false"],
+    "rpd_clip_thread.cu": ["-fmad=false"],
     "rpd_pairs.cu": ["-fmad=false"],
     "rpd_noalloc.cu": [],
     "rpd_mlp.cu": [],

@@ -631,6 +631,10 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
     p.cert_margin = cert_margin;
     p.pair_index = nullptr;
     p.n_work = n_pairs;
+    p.n_work_dev = nullptr;
+    p.centroid = c->centroid.ptr;
+    p.back_idx = nullptr;
+    p.back_count = c->scratch.ptr + 33;
     p.topo_hash = c->cfg.topology_hash ? c->topo_hash.ptr : nullptr;
     p.uncertified = nullptr;  // counted at the compaction, after every round
     p.nbr_bound = knn ? c->nbr_bound.ptr : nullptr;
@@ -641,7 +645,21 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
     p.ext_len = nullptr;
     p.ext_bound = nullptr;
     CK(cudaEventRecord(c->ev[kEvClipK0], st), "event");
-    if (n_pairs > 0) CK(launch_clip_cells(p, c->cfg.predicate_mode, certify, variant, blocks, warps, st), "clip");
+    if (n_pairs > 0) {
+      ClipParams pw = p;
+      if (clip_threads_takes(p, c->cfg.predicate_mode)) {
+        // scratch[33], [34]: the pairs left to the general kernel, and its
+        // queue's counter
+        CK(c->ext_idx.ensure((size_t)n_pairs), "alloc ext");
+        CK(cudaMemsetAsync(c->scratch.ptr + 33, 0, 2 * sizeof(unsigned long long), st), "memset");
+        p.back_idx = c->ext_idx.ptr;
+        CK(launch_clip_threads(p, c->cfg.predicate_mode, certify, c->num_sms, st), "clip");
+        pw.pair_index = c->ext_idx.ptr;
+        pw.n_work_dev = c->scratch.ptr + 33;
+        pw.work = c->scratch.ptr + 34;
+      }
+      CK(launch_clip_cells(pw, c->cfg.predicate_mode, certify, variant, blocks, warps, st), "clip");
+    }
     CK(cudaEventRecord(c->ev[kEvClipK1], st), "event");
     if ((p.site_klen || p.pair_klen) && n_pairs > 0) {
       // cells whose shortened list was not enough: clip them again whole

@@ -56,6 +56,16 @@ struct ClipParams {
   // optional indirection: work item w clips pair pair_index[w]
   const int32_t* pair_index;
   long long n_work;
+  const unsigned long long* n_work_dev;  // n_work on the device, or null
+  // clip_threads_kernel: centroids of the tets; the pairs it leaves to
+  // clip_cells_kernel (cells that outgrow a lane).  Set by its launch: the
+  // lanes of a warp that own cells, how many idle ones make it take new
+  // pairs, below how many scanning ones it clips, and how many undecided ones
+  // it decides together
+  const float4* centroid;
+  int32_t* back_idx;
+  unsigned long long* back_count;
+  int cell_lanes, refill_lanes, scan_lanes, und_lanes;
   unsigned long long* topo_hash;  // n_pairs canonical topology hashes, or null
   // completeness of the lists: every site missing from site s's base list
   // has a key >= nbr_bound[s] (INFINITY: the list holds every site); null =
@@ -142,6 +152,11 @@ int clip_blocks_per_sm(int pred_mode, int warps);
 int box_blocks_per_sm(int warps);
 // variant: 0 = no register cap (warps per block as given), 1 = at most 80
 // registers (6 blocks of 4 warps per SM), 2 = at most 64 (8 blocks of 4 warps)
+// one thread per cell, for the pairs of a first pass on whole base lists
+// (clip_threads_takes says which); what outgrows it lands in p.back_idx
+bool clip_threads_takes(const ClipParams& p, int pred_mode);
+cudaError_t launch_clip_threads(const ClipParams& p, int pred_mode, int certify, int num_sms,
+                                cudaStream_t st);
 cudaError_t launch_clip_cells(const ClipParams& p, int pred_mode, int certify, int variant,
                               int blocks, int warps, cudaStream_t st);
 int clip_blocks_per_sm_cert(int pred_mode, int certify, int warps, int variant);

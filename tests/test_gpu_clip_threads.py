@@ -1,0 +1,83 @@
+"""The thread-per-cell clipper (rpd_clip_thread.cu) against the FP64 path,
+which a warp per cell clips (and which the parity tests pin to the oracle):
+the same records byte for byte in site-id order, the same cells by canonical
+topology with certified lists, over list lengths that are and are not
+multiples of a group of four, few and many pairs per tet (cells that outgrow a
+lane go back to the warps), fewer pairs than lanes, ties, duplicated and
+unflagged sites, and lists with holes."""
+import numpy as np
+import pytest
+
+from libmat_gb300 import rpd
+from libmat_gb300 import workloads as W
+from tests.helpers import compare_cells
+
+pytestmark = pytest.mark.gpu
+
+MIN_PAIRS = 20000  # kThreadsPairs of rpd_clip_thread.cu
+
+
+def run(cfg, adj, pred, nbr=None, **kw):
+    with rpd.RPD(predicate_mode=pred, neighbor_source=rpd.NEIGH_KNN if nbr is None
+                 else rpd.NEIGH_USER, **kw) as r:
+        r.set_mesh(cfg["vert3d"], cfg["tets"], adj["v_adjs"], adj["e_adj6"], adj["f_adjs"],
+                   adj["f_ids"])
+        r.set_sites(cfg["sites"], cfg["flags"])
+        if nbr is not None:
+            r.set_neighbors(nbr)
+        st = r.compute()
+        return st, r.pair_headers(), r.cells(), r.topology_hashes()
+
+
+def case(kind):
+    if kind == "lattice":
+        return W.config_lattice(n=16, m=8)
+    if kind == "ellipsoid":
+        return W.config_ellipsoid(target_tets=40_000, n_site=2_000, seed=11)
+    n, sites = {"cube": (20, 2_000), "few_pairs": (10, 400), "dense": (9, 3_000)}[kind]
+    return W.config_small_cube(n=n, n_site=sites, seed=5)
+
+
+@pytest.mark.parametrize("kind,k", [("cube", 64), ("cube", 63), ("cube", 5), ("cube", 1),
+                                    ("few_pairs", 30), ("dense", 48), ("dense", 127),
+                                    ("lattice", 64), ("ellipsoid", 96)])
+def test_equals_fp64_path(kind, k):
+    cfg = case(kind)
+    adj = rpd.mesh_adjacency(cfg["vert3d"].shape[0], cfg["tets"])
+    a, ha, (_, pa), _ = run(cfg, adj, rpd.PRED_FP64, knn_k=k, exact_lists=False)
+    b, hb, (_, pb), _ = run(cfg, adj, rpd.PRED_FP32_FILTER, knn_k=k, exact_lists=False)
+    assert b.n_pairs == a.n_pairs >= MIN_PAIRS
+    assert np.array_equal(ha["flags"], hb["flags"])
+    assert np.array_equal(ha["volume"], hb["volume"], equal_nan=True)
+    assert compare_cells(ha, pa, hb, pb) == 0
+
+
+@pytest.mark.parametrize("kind,k", [("cube", 64), ("dense", 33), ("ellipsoid", 128)])
+def test_certified_cells_equal_fp64_path(kind, k):
+    cfg = case(kind)
+    adj = rpd.mesh_adjacency(cfg["vert3d"].shape[0], cfg["tets"])
+    a, ha, _, ta = run(cfg, adj, rpd.PRED_FP64, knn_k=k, certify=True)
+    b, hb, _, tb = run(cfg, adj, rpd.PRED_FP32_FILTER, knn_k=k, certify=True)
+    assert b.n_pairs == a.n_pairs >= MIN_PAIRS
+    assert a.n_uncertified == b.n_uncertified == 0
+    assert np.array_equal(ha["status"], hb["status"])
+    assert np.array_equal(ta, tb)
+
+
+def test_user_lists_with_holes_duplicates_and_unflagged_sites():
+    cfg = case("cube")
+    adj = rpd.mesh_adjacency(cfg["vert3d"].shape[0], cfg["tets"])
+    rng = np.random.default_rng(3)
+    cfg["sites"][100:140] = cfg["sites"][200:240]  # the same sphere twice
+    cfg["flags"][rng.choice(2_000, 300, replace=False)] = 0
+    with rpd.RPD(knn_k=50, exact_lists=False) as r:
+        r.set_mesh(cfg["vert3d"], cfg["tets"], adj["v_adjs"], adj["e_adj6"], adj["f_adjs"],
+                   adj["f_ids"])
+        r.set_sites(cfg["sites"], cfg["flags"])
+        r.compute()
+        nbr = r.neighbor_lists(2_000)
+    nbr[rng.integers(0, 2_000, 400), rng.integers(0, 50, 400)] = -1  # a list ends at its hole
+    a, ha, (_, pa), _ = run(cfg, adj, rpd.PRED_FP64, nbr=nbr)
+    b, hb, (_, pb), _ = run(cfg, adj, rpd.PRED_FP32_FILTER, nbr=nbr)
+    assert b.n_pairs == a.n_pairs >= MIN_PAIRS
+    assert compare_cells(ha, pa, hb, pb) == 0
