@@ -733,65 +733,6 @@ __device__ __forceinline__ int finish_list(const WarpCell& c, int nb_v, ListMeta
   return cert_holds(bound, R, margin) ? 0 : 1;
 }
 
-// ------------------------------------------------------------------------
-// FP64-accurate reconstruction of the emitted cell
-// ------------------------------------------------------------------------
-// The float planes above decide the topology exactly as the reference does.
-// The coordinates reported for the surviving vertices are rebuilt from the
-// FP64 inputs instead: every plane is recomputed in the frame centred on the
-// seed S, from double-float copies of the FP64 mesh vertices and sites
-// (hi + lo, about 48 bits), and each vertex -- the intersection of its three
-// planes, by Cramer's rule as in compute_vertex_coordinates
-// (convex_cell.cu:319-351) -- is solved in double-float arithmetic on the
-// FP32 pipe, then translated back by S and rounded to FP64 with one FP64
-// add.  The cell volume uses the reference's per-vertex decomposition into
-// six tets (convex_cell.cu:986-1069) in FP32, about a point of the cell
-// (small coordinates, no cancellation against the scene's extent).
-
-__device__ __forceinline__ df dmul3(df a, df b, df c) { return df_mul(df_mul(a, b), c); }
-
-// 2x2 minor b_p c_q - b_q c_p
-__device__ __forceinline__ df minor2(df bp, df bq, df cp, df cq) {
-  return df_sub_s(df_mul(bp, cq), df_mul(bq, cp));
-}
-
-__device__ __forceinline__ float3 f3sub(float3 a, float3 b) {
-  return make_float3(a.x - b.x, a.y - b.y, a.z - b.z);
-}
-__device__ __forceinline__ float f3dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ float3 f3cross(float3 a, float3 b) {
-  return make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-}
-__device__ __forceinline__ float3 f3axpy(float a, float3 x, float3 y) {
-  return make_float3(a * x.x + y.x, a * x.y + y.y, a * x.z + y.z);
-}
-__device__ __forceinline__ float det3f(float3 a, float3 b, float3 c) { return f3dot(a, f3cross(b, c)); }
-
-// foot of the origin O = (0,0,0) on the plane n.x + d = 0
-__device__ __forceinline__ float3 face_foot(float3 n, float d) {
-  const float n2 = f3dot(n, n);
-  const float lam = n2 > 0.f ? __fdividef(d, n2) : 0.f;
-  return make_float3(-lam * n.x, -lam * n.y, -lam * n.z);
-}
-
-// signed volume of one vertex's six flag tets, origin O = (0,0,0): feet of
-// O on the three faces (given) and on the three edge lines through A.  The
-// volume is reported in FP32, so the quotients use the fast division.
-__device__ float vertex_volume_f(float3 A, const float3* n, const float3* foot) {
-  float3 P[6];
-  for (int i = 0; i < 3; ++i) P[2 * i] = foot[i];
-  for (int i = 0; i < 3; ++i) {
-    float3 t = f3cross(n[i], n[(i + 1) % 3]);
-    float t2 = f3dot(t, t);
-    float lam = t2 > 0.f ? __fdividef(f3dot(t, A), t2) : 0.f;
-    P[2 * i + 1] = f3axpy(-lam, t, A);
-  }
-  float3 mA = make_float3(-A.x, -A.y, -A.z);
-  float v = 0.f;
-  for (int i = 0; i < 6; ++i) v -= det3f(f3sub(P[i], A), f3sub(P[(i + 1) % 6], A), mA);
-  return v * (1.0f / 6.0f);
-}
-
 // intersection of three float planes, double-float Cramer (box kernel):
 // per coordinate a float interval [lo, hi] around the double-float value
 __device__ void vertex_of_float_planes(float4 a4, float4 b4, float4 c4, float* lo, float* hi) {
@@ -813,195 +754,6 @@ __device__ void vertex_of_float_planes(float4 a4, float4 b4, float4 c4, float* l
     lo[k] = __fadd_rd(X[k].hi, X[k].lo);
     hi[k] = __fadd_ru(X[k].hi, X[k].lo);
   }
-}
-
-// vertex (X, Y, Z) of the three seed-frame double-float planes pa, pb, pc
-template <class Cell>
-__device__ __forceinline__ void cell_vertex(const Cell& c, int pa, int pb, int pc, df& X,
-                                            df& Y, df& Z) {
-  df ax = c.u.g.n[pa][0], ay = c.u.g.n[pa][1], az = c.u.g.n[pa][2], aw = c.u.g.d[pa];
-  df bx = c.u.g.n[pb][0], by = c.u.g.n[pb][1], bz = c.u.g.n[pb][2], bw = c.u.g.d[pb];
-  df cx = c.u.g.n[pc][0], cy = c.u.g.n[pc][1], cz = c.u.g.n[pc][2], cw = c.u.g.d[pc];
-  df mxy = minor2(bx, by, cx, cy), mxz = minor2(bx, bz, cx, cz), mxw = minor2(bx, bw, cx, cw);
-  df myz = minor2(by, bz, cy, cz), myw = minor2(by, bw, cy, cw), mzw = minor2(bz, bw, cz, cw);
-  df Dw = df_add_s(df_sub_s(df_mul(ax, myz), df_mul(ay, mxz)), df_mul(az, mxy));
-  df Dx = df_add_s(df_sub_s(df_mul(ay, mzw), df_mul(az, myw)), df_mul(aw, myz));
-  df Dy = df_add_s(df_sub_s(df_mul(ax, mzw), df_mul(az, mxw)), df_mul(aw, mxz));
-  df Dz = df_add_s(df_sub_s(df_mul(ax, myw), df_mul(ay, mxw)), df_mul(aw, mxy));
-  df inv = df_recip(Dw);
-  X = df_neg(df_mul(Dx, inv));
-  Y = df_mul(Dy, inv);
-  Z = df_neg(df_mul(Dz, inv));
-}
-
-template <class Cell>
-__device__ __forceinline__ float vertex_volume_about(const Cell& c, uchar4 tr, df X, df Y,
-                                                     df Z, float3 O) {
-  float3 A = make_float3(df_sub_s(X, df_make(O.x, 0.f)).hi, df_sub_s(Y, df_make(O.y, 0.f)).hi,
-                         df_sub_s(Z, df_make(O.z, 0.f)).hi);
-  const int pl[3] = {tr.x, tr.y, tr.z};
-  float3 nn[3], ft[3];
-  for (int k = 0; k < 3; ++k) {
-    nn[k] = make_float3(c.u.g.n[pl[k]][0].hi, c.u.g.n[pl[k]][1].hi, c.u.g.n[pl[k]][2].hi);
-    ft[k] = c.u.g.foot[pl[k]];
-  }
-  return vertex_volume_f(A, nn, ft);
-}
-
-__device__ __forceinline__ df ldf(const float2* p) {
-  const float2 v = __ldg(p);
-  return df_make(v.x, v.y);
-}
-
-// exact float -> double widening with integer operations (IEEE-754 binary32
-// to binary64: same sign, exponent re-biased by 1023 - 127, fraction shifted
-// by 29 bits); zeros, subnormals, infinities and NaNs take the conversion
-// instruction
-__device__ __forceinline__ double widen(float f) {
-  const uint32_t u = __float_as_uint(f);
-  const uint32_t e = (u >> 23) & 0xffu;
-  if (e == 0u || e == 0xffu) return (double)f;
-  const uint64_t bits = ((uint64_t)(u >> 31) << 63) | ((uint64_t)(e + 896u) << 52) |
-                        ((uint64_t)(u & 0x7fffffu) << 29);
-  return __longlong_as_double((long long)bits);
-}
-
-// S + X (double-float) rounded to double: hi and lo widen exactly, one add
-__device__ __forceinline__ double df_translate(df S, df X) {
-  const df t = df_add_s(S, X);
-  return widen(t.hi) + widen(t.lo);
-}
-
-// float intersection of three planes (Cramer); used only as the origin of
-// the volume decomposition, so any point near the cell will do
-template <class Cell>
-__device__ float3 float_vertex(const Cell& c, uchar4 tr) {
-  const int pl[3] = {tr.x, tr.y, tr.z};
-  float a[3][4];
-  for (int k = 0; k < 3; ++k) {
-    a[k][0] = c.u.g.n[pl[k]][0].hi;
-    a[k][1] = c.u.g.n[pl[k]][1].hi;
-    a[k][2] = c.u.g.n[pl[k]][2].hi;
-    a[k][3] = c.u.g.d[pl[k]].hi;
-  }
-  // n_k . x = -d_k
-  const float3 n0 = make_float3(a[0][0], a[0][1], a[0][2]);
-  const float3 n1 = make_float3(a[1][0], a[1][1], a[1][2]);
-  const float3 n2 = make_float3(a[2][0], a[2][1], a[2][2]);
-  const float3 c12 = f3cross(n1, n2), c20 = f3cross(n2, n0), c01 = f3cross(n0, n1);
-  const float det = f3dot(n0, c12);
-  const float s = -1.0f / det;
-  float3 x = make_float3(s * (a[0][3] * c12.x + a[1][3] * c20.x + a[2][3] * c01.x),
-                         s * (a[0][3] * c12.y + a[1][3] * c20.y + a[2][3] * c01.y),
-                         s * (a[0][3] * c12.z + a[1][3] * c20.z + a[2][3] * c01.z));
-  if (!(isfinite(x.x) && isfinite(x.y) && isfinite(x.z))) x = make_float3(0.f, 0.f, 0.f);
-  return x;
-}
-
-// writes xyz[3 * nb_v] and returns the cell volume; c holds the cell's
-// id2 and ver, c.u.g is filled here.  W lanes (a whole warp or a half) work
-// on the cell; lane is 0..W-1.  Every lane of the warp calls this the same
-// number of times (its __syncwarp and shuffles span the warp); a lane group
-// with no cell passes active = false.
-template <int W, class Cell>
-__device__ double cell_geometry(Cell& c, bool active, int nb_v, int nb_p, const float2* face2,
-                                const float2* site2, int tet, int sid, int lane, double* xyz) {
-  df Sx = df_make(0.f, 0.f), Sy = Sx, Sz = Sx, Sw = Sx;
-  if (active) {
-    const float2* S2 = site2 + 4 * (long long)sid;
-    Sx = ldf(S2);
-    Sy = ldf(S2 + 1);
-    Sz = ldf(S2 + 2);
-    Sw = ldf(S2 + 3);
-  } else {
-    nb_v = nb_p = 0;
-  }
-  for (int i = lane; i < nb_p; i += W) {
-    df nx, ny, nz, d;
-    if (i < 4) {
-      // the tet's face plane (FP64, once per mesh), moved to the seed frame:
-      // d' = d + n . S
-      const float2* f = face2 + 16 * (long long)tet + 4 * i;
-      nx = ldf(f);
-      ny = ldf(f + 1);
-      nz = ldf(f + 2);
-      d = df_add_s(ldf(f + 3), df_add_s(df_add_s(df_mul(nx, Sx), df_mul(ny, Sy)), df_mul(nz, Sz)));
-    } else {
-      const int2 id = c.id2[i];
-      const int other = id.x == sid ? id.y : id.x;
-      const float2* B = site2 + 4 * (long long)other;
-      // bisector in the seed frame: n = S - B, d = (|n|^2 + wS - wB) / 2
-      nx = df_sub_s(Sx, ldf(B));
-      ny = df_sub_s(Sy, ldf(B + 1));
-      nz = df_sub_s(Sz, ldf(B + 2));
-      const df n2 = df_add_s(df_add_s(df_mul(nx, nx), df_mul(ny, ny)), df_mul(nz, nz));
-      d = df_add_s(n2, df_sub_s(Sw, ldf(B + 3)));
-      d = df_make(0.5f * d.hi, 0.5f * d.lo);
-    }
-    c.u.g.n[i][0] = nx;
-    c.u.g.n[i][1] = ny;
-    c.u.g.n[i][2] = nz;
-    c.u.g.d[i] = d;
-  }
-  __syncwarp();
-  // volume origin O near the cell (its vertex 0, in float): the
-  // decomposition's terms then scale with the cell's own size
-  const float3 O = active ? float_vertex(c, c.ver[0]) : make_float3(0.f, 0.f, 0.f);
-  for (int i = lane; i < nb_p; i += W) {
-    const df n0 = c.u.g.n[i][0], n1 = c.u.g.n[i][1], n2 = c.u.g.n[i][2];
-    const df dc = df_add_s(c.u.g.d[i], df_add_s(df_add_s(df_mul(n0, df_make(O.x, 0.f)),
-                                                   df_mul(n1, df_make(O.y, 0.f))),
-                                            df_mul(n2, df_make(O.z, 0.f))));
-    c.u.g.foot[i] = face_foot(make_float3(n0.hi, n1.hi, n2.hi), dc.hi);
-  }
-  __syncwarp();
-  float vol = 0.f;
-  for (int v = lane; v < nb_v; v += W) {
-    const uchar4 tr = c.ver[v];
-    df X, Y, Z;
-    cell_vertex(c, tr.x, tr.y, tr.z, X, Y, Z);
-    xyz[3 * v] = df_translate(Sx, X);
-    xyz[3 * v + 1] = df_translate(Sy, Y);
-    xyz[3 * v + 2] = df_translate(Sz, Z);
-    vol += vertex_volume_about(c, tr, X, Y, Z, O);
-  }
-  for (int o = W / 2; o > 0; o >>= 1) vol += __shfl_xor_sync(0xffffffffu, vol, o);
-  return (double)vol;
-}
-
-// canonical topology of a cell, independent of the clipping order: the sum
-// over its vertices of a hash of the sorted face keys (clip_id2) of the
-// vertex's three planes and its #adjacent cells (splitmix64 mixing, Steele,
-// Lea and Flood, OOPSLA 2014).  Planes that clipped intermediate vertices and
-// no longer bound the cell appear in no vertex, so they do not count.
-__device__ __forceinline__ uint64_t mix64(uint64_t z) {
-  z += 0x9e3779b97f4a7c15ull;
-  z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
-  z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
-  return z ^ (z >> 31);
-}
-
-__device__ __forceinline__ uint64_t face_key(int2 id) {
-  return ((uint64_t)(uint32_t)id.x << 32) | (uint32_t)id.y;
-}
-
-template <int W, class Cell>
-__device__ uint64_t cell_topology_hash(const Cell& c, int nb_v, int lane) {
-  uint64_t h = 0;
-  for (int v = lane; v < nb_v; v += W) {
-    uchar4 t = c.ver[v];
-    uint64_t a = face_key(c.id2[t.x]), b = face_key(c.id2[t.y]), d = face_key(c.id2[t.z]), x;
-    if (a > b) { x = a; a = b; b = x; }
-    if (b > d) { x = b; b = d; d = x; }
-    if (a > b) { x = a; a = b; b = x; }
-    uint64_t hv = mix64(a);
-    hv = mix64(hv ^ b);
-    hv = mix64(hv ^ d);
-    hv = mix64(hv ^ (uint64_t)t.w);
-    h += hv;
-  }
-  for (int o = W / 2; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
-  return h;
 }
 
 // MINB > 0 caps registers so that MINB blocks of 128 threads fit on an SM
@@ -1220,119 +972,6 @@ __global__ void __launch_bounds__(128) recheck_cells_kernel(RecheckParams p) {
 
 cudaError_t launch_recheck_cells(const RecheckParams& p, int num_sms, cudaStream_t st) {
   recheck_cells_kernel<<<(unsigned)(num_sms * 16), 128, 0, st>>>(p);
-  note_launches(1);
-  return cudaGetLastError();
-}
-
-// ------------------------------------------------------------------------
-// epilogue: FP64-accurate coordinates and volume, canonical topology hash,
-// of every emitted cell, from its record (plane ids and dual triangles)
-// ------------------------------------------------------------------------
-// The clip kernel leaves these to a separate pass: it keeps the clip
-// kernel's code (and its instruction-cache footprint) to the topology
-// update, and every warp here runs the same short program.  The first four
-// planes of every record are the tet's faces, in order; the others are
-// bisectors with the site pair in id2.
-struct GeomCell {
-  struct {
-    struct {
-      df n[kMaxP][3];
-      df d[kMaxP];
-      float3 foot[kMaxP];
-    } g;
-  } u;
-  int2 id2[kMaxP];
-  uchar4 ver[kMaxT];
-};
-
-constexpr int kEpiWarps = 4;
-
-// two cells per warp, one per half-warp: most cells have fewer than 16
-// planes and few more vertices, so 16 lanes keep busier than 32
-__global__ void __launch_bounds__(kEpiWarps * 32) cell_epilogue_kernel(EpilogueParams p) {
-  __shared__ GeomCell cells[2 * kEpiWarps];
-  const int lane = threadIdx.x & 31;
-  const int half = lane >> 4, hl = lane & 15;
-  GeomCell& c = cells[2 * (threadIdx.x >> 5) + half];
-  const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long base = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2;
-       base < p.n_pairs; base += 2 * n_warps) {
-    const long long q = base + half;
-    rpd_cell_header hd;
-    bool active = false;
-    if (q < p.n_pairs) {
-      hd = p.headers[q];
-      active = hd.status == kSuccess;
-      if (!active && p.topo_hash && hl == 0) p.topo_hash[q] = 0ull;
-    }
-    const int nb_v = active ? hd.nb_v : 0, nb_p = active ? hd.nb_p : 0;
-    uint8_t* rec = nullptr;
-    PayloadLayout L(nb_v, nb_p, active ? hd.nb_e : 0);
-    if (active) {
-      rec = p.payload + hd.offset;
-      for (int i = hl; i < nb_p; i += 16) c.id2[i] = reinterpret_cast<const int2*>(rec + L.id2)[i];
-      for (int i = hl; i < nb_v; i += 16) c.ver[i] = reinterpret_cast<const uchar4*>(rec + L.ver)[i];
-    }
-    __syncwarp();
-    double* xyz = active ? reinterpret_cast<double*>(rec + L.xyz) : nullptr;
-    double vol = 0.0;
-    if (p.geometry) {
-      vol = cell_geometry<16>(c, active, nb_v, nb_p, p.face2, p.site2, active ? hd.tet_id : 0,
-                              active ? hd.site_id : 0, hl, xyz);
-    } else if (active) {
-      for (int i = hl; i < 3 * nb_v; i += 16) xyz[i] = 0.0;
-    }
-    uint64_t th = 0;
-    if (p.topo_hash) th = cell_topology_hash<16>(c, nb_v, hl);
-    if (active && hl == 0) {
-      p.headers[q].volume = vol;
-      if (p.topo_hash) p.topo_hash[q] = th;
-    }
-    __syncwarp();
-  }
-}
-
-cudaError_t launch_cell_epilogue(const EpilogueParams& p, int num_sms, cudaStream_t st) {
-  if (p.n_pairs <= 0) return cudaSuccess;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cell_epilogue_kernel, kEpiWarps * 32, 0);
-  if (per_sm < 1) per_sm = 1;
-  const long long want = (p.n_pairs + 2 * kEpiWarps - 1) / (2 * kEpiWarps);
-  long long blocks = (long long)num_sms * per_sm * 4;
-  if (blocks > want) blocks = want;
-  cell_epilogue_kernel<<<(unsigned)blocks, kEpiWarps * 32, 0, st>>>(p);
-  note_launches(1);
-  return cudaGetLastError();
-}
-
-// face planes of every tet in FP64 (inward normals as tri2plane,
-// common_cuda.h:248-254: n = (b - a) x (e - a), d = -a . n), stored as
-// double-float (nx, ny, nz, d) per face
-__global__ void tet_face_planes_kernel(const double* vert, const int4* tets, int n_tet, float2* out) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_tet) return;
-  const int4 q = tets[t];
-  const int id[4] = {q.x, q.y, q.z, q.w};
-  for (int i = 0; i < 4; ++i) {
-    const double* a = vert + 3 * (long long)id[cFaceLv[i][0]];
-    const double* b = vert + 3 * (long long)id[cFaceLv[i][1]];
-    const double* e = vert + 3 * (long long)id[cFaceLv[i][2]];
-    const double ux = b[0] - a[0], uy = b[1] - a[1], uz = b[2] - a[2];
-    const double vx = e[0] - a[0], vy = e[1] - a[1], vz = e[2] - a[2];
-    const double nx = uy * vz - uz * vy, ny = uz * vx - ux * vz, nz = ux * vy - uy * vx;
-    const double d = -(a[0] * nx + a[1] * ny + a[2] * nz);
-    const double v[4] = {nx, ny, nz, d};
-    for (int k = 0; k < 4; ++k) {
-      const df x = df_from_double(v[k]);
-      out[16ll * t + 4 * i + k] = make_float2(x.hi, x.lo);
-    }
-  }
-}
-
-cudaError_t launch_tet_face_planes(const double* vert3d, const int4* tets, int n_tet, float2* out,
-                                   cudaStream_t st) {
-  if (n_tet <= 0) return cudaSuccess;
-  tet_face_planes_kernel<<<(n_tet + 255) / 256, 256, 0, st>>>(vert3d, tets, n_tet, out);
   note_launches(1);
   return cudaGetLastError();
 }

@@ -97,4 +97,9 @@ __device__ __forceinline__ df df_recip(df y) {
   return fast_two_sum(q, q2);
 }
 
+// 2x2 minor b_p c_q - b_q c_p
+__device__ __forceinline__ df minor2(df bp, df bq, df cp, df cq) {
+  return df_sub_s(df_mul(bp, cq), df_mul(bq, cp));
+}
+
 }  // namespace rpd
