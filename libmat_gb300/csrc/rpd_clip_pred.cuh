@@ -37,23 +37,36 @@ __device__ __forceinline__ float4 bisector_f(float4 S, float4 B) {
   return make_float4(dx, dy, dz, -dot / 2.f);
 }
 
-__device__ __forceinline__ double det4x4_ref(float4 p1, float4 p2, float4 p3,
-                                             float4 e) {
-  double a11 = p1.x, a12 = p2.x, a13 = p3.x, a14 = e.x;
-  double a21 = p1.y, a22 = p2.y, a23 = p3.y, a24 = e.y;
-  double a31 = p1.z, a32 = p2.z, a33 = p3.z, a34 = e.z;
-  double a41 = p1.w, a42 = p2.w, a43 = p3.w, a44 = e.w;
+// det4x4_ref(p1, p2, p3, e) = m234 e.x - m134 e.y + m124 e.z - m123 e.w: the
+// minors of the vertex's planes do not depend on e, and the reference rounds
+// them before e comes in
+struct Minors {
+  double m234, m134, m124, m123;
+};
+__device__ __forceinline__ Minors det4x4_minors(float4 p1, float4 p2, float4 p3) {
+  double a11 = p1.x, a12 = p2.x, a13 = p3.x;
+  double a21 = p1.y, a22 = p2.y, a23 = p3.y;
+  double a31 = p1.z, a32 = p2.z, a33 = p3.z;
+  double a41 = p1.w, a42 = p2.w, a43 = p3.w;
   double m12 = a21 * a12 - a11 * a22;
   double m13 = a31 * a12 - a11 * a32;
   double m14 = a41 * a12 - a11 * a42;
   double m23 = a31 * a22 - a21 * a32;
   double m24 = a41 * a22 - a21 * a42;
   double m34 = a41 * a32 - a31 * a42;
-  double m123 = m23 * a13 - m13 * a23 + m12 * a33;
-  double m124 = m24 * a13 - m14 * a23 + m12 * a43;
-  double m134 = m34 * a13 - m14 * a33 + m13 * a43;
-  double m234 = m34 * a23 - m24 * a33 + m23 * a43;
-  return (m234 * a14 - m134 * a24 + m124 * a34 - m123 * a44);
+  Minors m;
+  m.m123 = m23 * a13 - m13 * a23 + m12 * a33;
+  m.m124 = m24 * a13 - m14 * a23 + m12 * a43;
+  m.m134 = m34 * a13 - m14 * a33 + m13 * a43;
+  m.m234 = m34 * a23 - m24 * a33 + m23 * a43;
+  return m;
+}
+__device__ __forceinline__ double det4x4_of(const Minors& m, float4 e) {
+  double a14 = e.x, a24 = e.y, a34 = e.z, a44 = e.w;
+  return (m.m234 * a14 - m.m134 * a24 + m.m124 * a34 - m.m123 * a44);
+}
+__device__ __forceinline__ double det4x4_ref(float4 p1, float4 p2, float4 p3, float4 e) {
+  return det4x4_of(det4x4_minors(p1, p2, p3), e);
 }
 
 // float det3x3 of the three plane normals (convex_cell.cu:274-316, the w
