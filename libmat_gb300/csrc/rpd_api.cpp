@@ -281,7 +281,7 @@ void rpd_destroy(rpd_ctx* c) {
   c->nbr.release(); c->nbr_dist.release(); c->site_klen.release(); c->reclip_idx.release();
   c->topo_hash.release(); c->nbr_ref_tmp.release(); c->knn_status.release(); c->nbr_keys.release();
   c->nbr_bound.release(); c->site_need.release(); c->site_row.release(); c->ext_sites.release();
-  c->site_flag.release(); c->site_pos.release(); c->ext_idx.release(); c->ext_nbr.release();
+  c->sel_count.release(); c->ext_idx.release(); c->ext_nbr.release();
   c->ext_len.release();
   c->ext_keys.release(); c->ext_bound.release(); c->ext_off.release();
   c->s_cell_of.release(); c->s_cell_count.release(); c->s_cell_start.release();
@@ -293,7 +293,7 @@ void rpd_destroy(rpd_ctx* c) {
   c->pair_buf.release(); c->tet_count.release(); c->tet_offsets.release();
   c->tet_fill.release(); c->pair_site.release(); c->pair_tet.release();
   c->pair_headers.release(); c->cells.release(); c->payload.release();
-  c->flag_tmp.release(); c->pos_tmp.release(); c->scratch.release(); c->n_out.release();
+  c->scratch.release(); c->n_out.release();
   for (int i = 0; i < kEvCount; ++i)
     if (c->ev[i]) cudaEventDestroy(c->ev[i]);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -572,17 +572,24 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
   long long n_ext_sites = 0, n_cert_reclipped = 0;
   int n_ext_rounds = 0, ext_longest = 0;
   float ms_ext_lists = 0.f;
+  CK(c->sel_count.ensure(2), "alloc");
+  CK(c->cells.ensure((size_t)std::max<long long>(n_pairs, 1)), "alloc cells");
+  CK(c->n_out.ensure(1), "alloc");
   if (extend) {
     CK(c->site_need.ensure((size_t)n_site), "alloc");
     CK(c->site_row.ensure((size_t)n_site), "alloc");
     CK(c->ext_sites.ensure((size_t)n_site), "alloc");
-    CK(c->site_flag.ensure((size_t)n_site), "alloc");
-    CK(c->site_pos.ensure((size_t)n_site + 1), "alloc");
     CK(c->scan_tmp.ensure(scan_temp_ints(std::max<long long>(std::max<long long>(n_pairs, n_tet),
                                                              n_site)) + 16), "alloc");
   }
+  unsigned long long host_scratch[40];
+  long long n_cells = 0;
   for (int attempt = 0; attempt < 3; ++attempt) {
-    CK(cudaMemsetAsync(c->scratch.ptr + 28, 0, 4 * sizeof(unsigned long long), st), "memset");
+    // [0..3] cursors and predicate counts, [8..18] statuses, [28..34] counts
+    // of this attempt and queues
+    CK(cudaMemsetAsync(c->scratch.ptr, 0, 4 * sizeof(unsigned long long), st), "memset");
+    CK(cudaMemsetAsync(c->scratch.ptr + 8, 0, 11 * sizeof(unsigned long long), st), "memset");
+    CK(cudaMemsetAsync(c->scratch.ptr + 28, 0, 7 * sizeof(unsigned long long), st), "memset");
     if (extend) {
       CK(cudaMemsetAsync(c->site_need.ptr, 0, sizeof(unsigned int) * (size_t)n_site, st), "memset");
       CK(cudaMemsetAsync(c->site_row.ptr, 0xff, sizeof(int32_t) * (size_t)n_site, st), "memset");
@@ -593,7 +600,6 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
       ms_ext_lists = 0.f;
     }
     CK(c->payload.ensure((size_t)pcap), "alloc payload");
-    CK(cudaMemsetAsync(c->scratch.ptr, 0, 4 * sizeof(unsigned long long), st), "memset");
     ClipParams p;
     p.vert3f = c->vert3f.ptr;
     p.vert3d = c->vert3d.ptr;
@@ -651,7 +657,6 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
         // scratch[33], [34]: the pairs left to the general kernel, and its
         // queue's counter
         CK(c->ext_idx.ensure((size_t)n_pairs), "alloc ext");
-        CK(cudaMemsetAsync(c->scratch.ptr + 33, 0, 2 * sizeof(unsigned long long), st), "memset");
         p.back_idx = c->ext_idx.ptr;
         CK(launch_clip_threads(p, c->cfg.predicate_mode, certify, c->num_sms, st), "clip");
         pw.pair_index = c->ext_idx.ptr;
@@ -663,15 +668,12 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
     CK(cudaEventRecord(c->ev[kEvClipK1], st), "event");
     if ((p.site_klen || p.pair_klen) && n_pairs > 0) {
       // cells whose shortened list was not enough: clip them again whole
-      CK(c->flag_tmp.ensure((size_t)n_pairs + 1), "alloc");
-      CK(c->pos_tmp.ensure((size_t)n_pairs + 1), "alloc");
       CK(c->reclip_idx.ensure((size_t)n_pairs), "alloc");
-      CK(c->scan_tmp.ensure(scan_temp_ints(std::max<long long>(n_pairs, n_tet)) + 16), "alloc");
-      CK(select_pairs(c->pair_headers.ptr, n_pairs, kSecurityRadiusNotReached, c->flag_tmp.ptr,
-                      c->pos_tmp.ptr, c->scan_tmp.ptr, c->reclip_idx.ptr, st), "select");
+      CK(select_pairs(c->pair_headers.ptr, n_pairs, kSecurityRadiusNotReached, c->scan_tmp.ptr,
+                      c->reclip_idx.ptr, c->sel_count.ptr, st), "select");
       int32_t n_re = 0;
       SmallReads rd(c, st);
-      CK(rd.add(&n_re, c->pos_tmp.ptr + n_pairs, sizeof(n_re)), "D2H");
+      CK(rd.add(&n_re, c->sel_count.ptr, sizeof(n_re)), "D2H");
       CK(rd.wait(), "reclip sync");
       c->n_reclipped = n_re;
       if (n_re > 0) {
@@ -691,18 +693,16 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
     CK(cudaEventRecord(c->ev[kEvExt0], st), "event");
     // (scratch[32]: cells still flagged after a recheck, compacted into
     // ext_idx; the selection's count is read on the device)
-    CK(c->flag_tmp.ensure((size_t)n_pairs + 1), "alloc");
-    CK(c->pos_tmp.ensure((size_t)n_pairs + 1), "alloc");
     CK(c->reclip_idx.ensure((size_t)std::max<long long>(n_pairs, 1)), "alloc");
     CK(c->ext_idx.ensure((size_t)std::max<long long>(n_pairs, 1)), "alloc");
     auto recheck = [&](bool rows) -> rpd_status {
-      CK(select_uncertified(c->pair_headers.ptr, n_pairs, c->flag_tmp.ptr, c->pos_tmp.ptr,
-                            c->scan_tmp.ptr, c->reclip_idx.ptr, st), "select cells");
+      CK(select_uncertified(c->pair_headers.ptr, n_pairs, c->scan_tmp.ptr, c->reclip_idx.ptr,
+                            c->sel_count.ptr, st), "select cells");
       CK(cudaMemsetAsync(c->scratch.ptr + 32, 0, sizeof(unsigned long long), st), "memset");
       RecheckParams rp;
       rp.headers = c->pair_headers.ptr;
       rp.idx = c->reclip_idx.ptr;
-      rp.n_dev = c->pos_tmp.ptr + n_pairs;
+      rp.n_dev = c->sel_count.ptr;
       rp.payload = c->payload.ptr;
       rp.site4f = c->site4f.ptr;
       rp.site_row = rows ? c->site_row.ptr : nullptr;
@@ -724,12 +724,12 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
     // those cells are clipped again; a round's re-clip can leave a cell
     // uncertified (its list was cut at kExtK), which the next round takes up
     for (int round = 0; extend && n_pairs > 0 && round < kExtRounds; ++round) {
-      CK(select_sites(c->site_need.ptr, n_site, c->site_flag.ptr, c->site_pos.ptr, c->scan_tmp.ptr,
-                      c->ext_sites.ptr, st), "select sites");
+      CK(select_sites(c->site_need.ptr, n_site, c->scan_tmp.ptr, c->ext_sites.ptr,
+                      c->sel_count.ptr + 1, st), "select sites");
       int32_t n_f = 0;
       unsigned long long n_flag = 0;
       SmallReads rd(c, st);
-      CK(rd.add(&n_f, c->site_pos.ptr + n_site, sizeof(n_f)), "D2H");
+      CK(rd.add(&n_f, c->sel_count.ptr + 1, sizeof(n_f)), "D2H");
       CK(rd.add(&n_flag, c->scratch.ptr + 32, sizeof(n_flag)), "D2H");
       CK(rd.wait(), "extend sync");
       if (round > 0) {
@@ -822,19 +822,8 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
     }
     CK(cudaEventRecord(c->ev[kEvExt1], st), "event");
     c->ext_valid = extend;
-    unsigned long long cur = 0;
-    SmallReads rd(c, st);
-    CK(rd.add(&cur, c->scratch.ptr, sizeof(cur)), "D2H");
-    CK(rd.wait(), "clip sync");
-    c->payload_bytes = (long long)cur;
-    if ((long long)cur <= (long long)c->payload.cap) break;
-    pcap = (long long)cur + (long long)cur / 8 + (1 << 20);
-    if (attempt == 2) return fail(c, RPD_ERR_CAPACITY, "rpd_compute: payload buffer");
-  }
-  c->payload_cap_hint = std::max<long long>(c->payload_cap_hint, c->payload_bytes + c->payload_bytes / 8 + (1 << 20));
-  // coordinates, volumes and topology hashes of the emitted cells
-  CK(cudaEventRecord(c->ev[kEvEpi0], st), "event");
-  {
+    // coordinates, volumes and topology hashes of the emitted cells
+    CK(cudaEventRecord(c->ev[kEvEpi0], st), "event");
     EpilogueParams ep;
     ep.headers = c->pair_headers.ptr;
     ep.n_pairs = n_pairs;
@@ -844,28 +833,25 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
     ep.geometry = c->cfg.compute_geometry;
     ep.topo_hash = c->cfg.topology_hash ? c->topo_hash.ptr : nullptr;
     CK(launch_cell_epilogue(ep, c->num_sms, st), "epilogue");
-  }
-  CK(cudaEventRecord(c->ev[kEvClip], st), "event");
-
-  // ---- compaction
-  CK(c->cells.ensure((size_t)std::max<long long>(n_pairs, 1)), "alloc cells");
-  CK(c->flag_tmp.ensure((size_t)n_pairs + 1), "alloc");
-  CK(c->pos_tmp.ensure((size_t)n_pairs + 1), "alloc");
-  CK(c->scan_tmp.ensure(scan_temp_ints(std::max<long long>(n_pairs, n_tet)) + 16), "alloc");
-  CK(c->n_out.ensure(1), "alloc");
-  CK(cudaMemsetAsync(c->scratch.ptr + 31, 0, sizeof(unsigned long long), st), "memset");
-  CK(compact_cells(c->pair_headers.ptr, n_pairs, c->flag_tmp.ptr, c->pos_tmp.ptr, c->scan_tmp.ptr,
-                   c->cells.ptr, c->n_out.ptr, c->scratch.ptr + 8, st, c->scratch.ptr + 31),
-     "compact");
-  CK(cudaEventRecord(c->ev[kEvEnd], st), "event");
-  unsigned long long host_scratch[40];
-  long long n_cells = 0;
-  {
+    CK(cudaEventRecord(c->ev[kEvClip], st), "event");
+    // ---- compaction, and one read of everything: a payload buffer that was
+    // too small (cells lost to it carry a status of their own, which the
+    // passes above leave alone) runs the attempt again
+    CK(compact_cells(c->pair_headers.ptr, n_pairs, c->scan_tmp.ptr, c->cells.ptr, c->n_out.ptr,
+                     c->scratch.ptr + 8, st, c->scratch.ptr + 31),
+       "compact");
+    CK(cudaEventRecord(c->ev[kEvEnd], st), "event");
     SmallReads rd(c, st);
     CK(rd.add(host_scratch, c->scratch.ptr, sizeof(host_scratch)), "D2H");
     CK(rd.add(&n_cells, c->n_out.ptr, sizeof(n_cells)), "D2H");
     CK(rd.wait(), "compute sync");
+    const long long cur = (long long)host_scratch[0];
+    c->payload_bytes = cur;
+    if (cur <= (long long)c->payload.cap) break;
+    pcap = cur + cur / 8 + (1 << 20);
+    if (attempt == 2) return fail(c, RPD_ERR_CAPACITY, "rpd_compute: payload buffer");
   }
+  c->payload_cap_hint = std::max<long long>(c->payload_cap_hint, c->payload_bytes + c->payload_bytes / 8 + (1 << 20));
   c->n_cells = n_cells;
   c->tet_k = (int)reinterpret_cast<int32_t*>(host_scratch + 5)[0];
   c->has_result = true;
@@ -2218,10 +2204,10 @@ rpd_status rpd_mlp_collect(rpd_ctx* c, int64_t max_samples, int64_t* n_total) {
   const long long n_pairs = c->n_pairs;
   if (n_pairs > 0 && max_samples > 0) {
     CK(c->reclip_idx.ensure((size_t)n_pairs), "alloc");
-    CK(select_pairs(c->pair_headers.ptr, n_pairs, kSuccess, c->flag_tmp.ptr, c->pos_tmp.ptr,
-                    c->scan_tmp.ptr, c->reclip_idx.ptr, st), "select");
+    CK(select_pairs(c->pair_headers.ptr, n_pairs, kSuccess, c->scan_tmp.ptr, c->reclip_idx.ptr,
+                    c->sel_count.ptr, st), "select");
     int32_t n_sel = 0;
-    CK(cudaMemcpyAsync(&n_sel, c->pos_tmp.ptr + n_pairs, sizeof(n_sel), cudaMemcpyDeviceToHost, st), "D2H");
+    CK(cudaMemcpyAsync(&n_sel, c->sel_count.ptr, sizeof(n_sel), cudaMemcpyDeviceToHost, st), "D2H");
     CK(cudaStreamSynchronize(st), "collect sync");
     if (n_sel > 0) {
       // every stride-th emitted cell in (tet, site) order

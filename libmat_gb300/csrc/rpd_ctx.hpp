@@ -140,7 +140,8 @@ struct rpd_ctx {
   DevBuf<float> nbr_bound;          // n_site
   DevBuf<unsigned int> site_need;   // n_site: radius bound (float bits), 0 = none
   DevBuf<int32_t> site_row;         // n_site: extended row, -1 = base list
-  DevBuf<int32_t> ext_sites, site_flag, site_pos, ext_idx;
+  DevBuf<int32_t> ext_sites, ext_idx;
+  DevBuf<int32_t> sel_count;  // pairs and sites selected last
   DevBuf<int32_t> ext_nbr, ext_len;
   DevBuf<float> ext_keys, ext_bound;
   DevBuf<long long> ext_off;
@@ -229,7 +230,6 @@ struct rpd_ctx {
   DevBuf<int32_t> d2m_closest;
   DevBuf<unsigned int> d2m_bad;
   DevBuf<uint8_t> payload;
-  DevBuf<int32_t> flag_tmp, pos_tmp;
   DevBuf<unsigned long long> scratch;  // [0] payload cursor [1] work [2..3] counters
                                        // [4] pair cursor [8..18] status hist
                                        // [32] cells still uncertified

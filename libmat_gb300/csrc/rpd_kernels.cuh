@@ -160,10 +160,10 @@ cudaError_t launch_clip_threads(const ClipParams& p, int pred_mode, int certify,
 cudaError_t launch_clip_cells(const ClipParams& p, int pred_mode, int certify, int variant,
                               int blocks, int warps, cudaStream_t st);
 int clip_blocks_per_sm_cert(int pred_mode, int certify, int warps, int variant);
-// indices of the pairs whose header status equals `status`
-cudaError_t select_pairs(const rpd_cell_header* h, long long n, int status, int32_t* flag_tmp,
-                         int32_t* pos_tmp, int32_t* scan_tmp, int32_t* idx_out,
-                         cudaStream_t st);
+// indices of the pairs whose header status equals `status`, and their count
+// (here and below scan_tmp holds scan_temp_ints(n) ints)
+cudaError_t select_pairs(const rpd_cell_header* h, long long n, int status, int32_t* scan_tmp,
+                         int32_t* idx_out, int32_t* count_out, cudaStream_t st);
 cudaError_t launch_site_box(const BoxParams& p, int blocks, int warps, cudaStream_t st);
 
 // ---- uniform grids, kNN, candidate pairs, scans (rpd_pairs.cu)
@@ -290,17 +290,15 @@ cudaError_t pairs_to_csr(const int2* pair_buf, long long n_pairs, int n_tet,
 // compaction of emitted cells (status success) in pair order; n_uncert
 // (optional) counts the emitted cells flagged RPD_CELL_UNCERTIFIED
 cudaError_t compact_cells(const rpd_cell_header* pair_headers, long long n_pairs,
-                          int32_t* flag_tmp, int32_t* pos_tmp, int32_t* scan_tmp,
-                          rpd_cell_header* out, long long* n_out_dev,
+                          int32_t* scan_tmp, rpd_cell_header* out, long long* n_out_dev,
                           unsigned long long* status_hist, cudaStream_t st,
                           unsigned long long* n_uncert = nullptr);
-// indices of the pairs whose header carries RPD_CELL_UNCERTIFIED
-cudaError_t select_uncertified(const rpd_cell_header* h, long long n, int32_t* flag_tmp,
-                               int32_t* pos_tmp, int32_t* scan_tmp, int32_t* idx_out,
-                               cudaStream_t st);
-// sites with site_need != 0, ascending (idx_out), their count at pos_tmp[n]
-cudaError_t select_sites(const unsigned int* site_need, int n, int32_t* flag_tmp,
-                         int32_t* pos_tmp, int32_t* scan_tmp, int32_t* idx_out, cudaStream_t st);
+// indices of the pairs whose header carries RPD_CELL_UNCERTIFIED, their count
+cudaError_t select_uncertified(const rpd_cell_header* h, long long n, int32_t* scan_tmp,
+                               int32_t* idx_out, int32_t* count_out, cudaStream_t st);
+// sites with site_need != 0, ascending, and their count
+cudaError_t select_sites(const unsigned int* site_need, int n, int32_t* scan_tmp,
+                         int32_t* idx_out, int32_t* count_out, cudaStream_t st);
 // extended rows row0 + f (f < n) of the sites sites[f]: site_row[sites[f]] =
 // row0 + f, ext_off[row0 + f] = off0 + f * stride
 cudaError_t assign_rows(const int32_t* sites, int n, int row0, long long off0, int stride,

@@ -41,53 +41,11 @@ int take_launches() {
 // ------------------------------------------------------------------------
 // scan
 // ------------------------------------------------------------------------
-constexpr int kScanBlock = 1024;
-
-size_t scan_temp_ints(long long n) { return (size_t)((n + kScanBlock - 1) / kScanBlock) + 1; }
-
-__global__ void scan_reduce_kernel(const int32_t* in, long long n, int32_t* block_sums) {
-  long long i = (long long)blockIdx.x * kScanBlock + threadIdx.x;
-  int v = i < n ? in[i] : 0;
-  int tot;
-  block_excl_scan<int>(v, &tot);
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
-}
-
-__global__ void scan_blocksums_kernel(int32_t* sums, int nb) {
-  int carry = 0;
-  for (int base = 0; base < nb; base += kScanBlock) {
-    int i = base + threadIdx.x;
-    int v = i < nb ? sums[i] : 0;
-    int tot;
-    int ex = block_excl_scan<int>(v, &tot);
-    if (i < nb) sums[i] = ex + carry;
-    carry += tot;
-  }
-  if (threadIdx.x == 0) sums[nb] = carry;
-}
-
-__global__ void scan_apply_kernel(const int32_t* in, long long n, const int32_t* block_sums,
-                                  int nb, int32_t* out) {
-  long long i = (long long)blockIdx.x * kScanBlock + threadIdx.x;
-  int v = i < n ? in[i] : 0;
-  int ex = block_excl_scan<int>(v, nullptr);
-  if (i < n) out[i] = ex + block_sums[blockIdx.x];
-  if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = block_sums[nb];
-}
+size_t scan_temp_ints(long long n) { return (size_t)((n + kKeepTile - 1) / kKeepTile) + 1; }
 
 cudaError_t scan_exclusive(const int32_t* in, int32_t* out, long long n, int32_t* temp,
                            cudaStream_t st) {
-  int nb = (int)((n + kScanBlock - 1) / kScanBlock);
-  if (nb == 0) {
-    return cudaMemsetAsync(out, 0, sizeof(int32_t), st);
-  }
-  scan_reduce_kernel<<<nb, kScanBlock, 0, st>>>(in, n, temp);
-  note_launches(1);
-  scan_blocksums_kernel<<<1, kScanBlock, 0, st>>>(temp, nb);
-  note_launches(1);
-  scan_apply_kernel<<<nb, kScanBlock, 0, st>>>(in, n, temp, nb, out);
-  note_launches(1);
-  return cudaGetLastError();
+  return scan_counts<int32_t>(in, out, n, temp, st);
 }
 
 // ------------------------------------------------------------------------
@@ -119,6 +77,8 @@ __global__ void bin_points_kernel(const float4* pts, int n, Grid g, int32_t* cel
   if (cell_rmax) atomicMax(reinterpret_cast<unsigned int*>(cell_rmax) + c, __float_as_uint(p.w));
 }
 
+// the cells' items; their order within a cell is not kept (the pair list is
+// sorted per tet, the neighbour lists by key and id)
 __global__ void fill_cells_kernel(int n, const int32_t* cell_of, const int32_t* cell_start,
                                   int32_t* cell_fill, int32_t* cell_items) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -129,22 +89,6 @@ __global__ void fill_cells_kernel(int n, const int32_t* cell_of, const int32_t* 
   cell_items[cell_start[c] + slot] = i;
 }
 
-// insertion sort of each cell's item list (short lists): deterministic order
-__global__ void sort_cells_kernel(int n_cells, const int32_t* cell_start, int32_t* items) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n_cells) return;
-  int b = cell_start[c], e = cell_start[c + 1];
-  for (int i = b + 1; i < e; ++i) {
-    int v = items[i];
-    int j = i - 1;
-    while (j >= b && items[j] > v) {
-      items[j + 1] = items[j];
-      --j;
-    }
-    items[j + 1] = v;
-  }
-}
-
 static cudaError_t grid_finish(int n, const Grid& g, const int32_t* cell_of, int32_t* cell_count,
                                int32_t* cell_start, int32_t* cell_fill, int32_t* cell_items,
                                int32_t* scan_tmp, cudaStream_t st) {
@@ -153,9 +97,6 @@ static cudaError_t grid_finish(int n, const Grid& g, const int32_t* cell_of, int
   if (err != cudaSuccess) return err;
   cudaMemsetAsync(cell_fill, 0, sizeof(int32_t) * n_cells, st);
   fill_cells_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, cell_of, cell_start, cell_fill, cell_items);
-  note_launches(1);
-  sort_cells_kernel<<<(int)((n_cells + 255) / 256), 256, 0, st>>>((int)n_cells, cell_start,
-                                                                 cell_items);
   note_launches(1);
   return cudaGetLastError();
 }
@@ -954,121 +895,104 @@ cudaError_t pairs_to_csr(const int2* pair_buf, long long n_pairs, int n_tet,
 // ------------------------------------------------------------------------
 // compaction
 // ------------------------------------------------------------------------
-__global__ void flag_cells_kernel(const rpd_cell_header* h, long long n, int32_t* flag,
-                                  unsigned long long* hist, unsigned long long* n_uncert) {
-  __shared__ unsigned int sh[12];
-  if (threadIdx.x < 12) sh[threadIdx.x] = 0;
-  __syncthreads();
-  long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) {
-    const rpd_cell_header hq = h[q];
-    const int s = hq.status;
-    flag[q] = s == kSuccess ? 1 : 0;
-    int b = (s >= 0 && s <= 8) ? s : (s == kPayloadFull ? 10 : 9);
-    atomicAdd(sh + b, 1u);
-    if (s == kSuccess && (hq.flags & RPD_CELL_UNCERTIFIED)) atomicAdd(sh + 11, 1u);
+// statuses counted on the way: hist[0..8], 9 other, 10 lost to a full
+// payload buffer; uncertified cells
+struct CountCells {
+  const rpd_cell_header* h;
+  unsigned long long* hist;
+  unsigned long long* n_uncert;
+  static __device__ unsigned int* bins() {
+    __shared__ unsigned int sh[12];
+    return sh;
   }
-  __syncthreads();
-  if (threadIdx.x < 11 && sh[threadIdx.x]) atomicAdd(hist + threadIdx.x, (unsigned long long)sh[threadIdx.x]);
-  if (threadIdx.x == 11 && n_uncert && sh[11]) atomicAdd(n_uncert, (unsigned long long)sh[11]);
-}
+  __device__ void begin() const {
+    if (threadIdx.x < 12) bins()[threadIdx.x] = 0;
+    __syncthreads();
+  }
+  __device__ bool operator()(long long q) const {
+    const int4 v = reinterpret_cast<const int4*>(h + q)[0];
+    const int s = v.z;
+    atomicAdd(bins() + ((s >= 0 && s <= 8) ? s : (s == kPayloadFull ? 10 : 9)), 1u);
+    if (s == kSuccess && (((uint32_t)v.w >> 24) & RPD_CELL_UNCERTIFIED)) atomicAdd(bins() + 11, 1u);
+    return s == kSuccess;
+  }
+  __device__ void end() const {
+    __syncthreads();
+    const unsigned int* sh = bins();
+    if (threadIdx.x < 11 && sh[threadIdx.x])
+      atomicAdd(hist + threadIdx.x, (unsigned long long)sh[threadIdx.x]);
+    if (threadIdx.x == 11 && n_uncert && sh[11])
+      atomicAdd(n_uncert, (unsigned long long)sh[11]);
+  }
+};
 
-__global__ void gather_cells_kernel(const rpd_cell_header* h, long long n, const int32_t* pos,
-                                    rpd_cell_header* out, long long* n_out) {
-  long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n && h[q].status == kSuccess) out[pos[q]] = h[q];
-  if (q == 0) *n_out = pos[n];
-}
+// a test without anything counted on the way
+template <class Test>
+struct Plain {
+  Test test;
+  __device__ void begin() const {}
+  __device__ bool operator()(long long q) const { return test(q); }
+  __device__ void end() const {}
+};
 
-cudaError_t compact_cells(const rpd_cell_header* pair_headers, long long n_pairs, int32_t* flag_tmp,
-                          int32_t* pos_tmp, int32_t* scan_tmp, rpd_cell_header* out,
-                          long long* n_out_dev, unsigned long long* status_hist, cudaStream_t st,
+struct HasStatus {
+  const rpd_cell_header* h;
+  int status;
+  __device__ bool operator()(long long q) const { return h[q].status == status; }
+};
+struct IsUncertified {
+  const rpd_cell_header* h;
+  __device__ bool operator()(long long q) const {
+    const int4 v = reinterpret_cast<const int4*>(h + q)[0];
+    return v.z == kSuccess && (((uint32_t)v.w >> 24) & RPD_CELL_UNCERTIFIED);
+  }
+};
+struct IsNeeded {
+  const unsigned int* need;
+  __device__ bool operator()(long long q) const { return need[q] != 0u; }
+};
+
+struct PutHeader {
+  const rpd_cell_header* h;
+  rpd_cell_header* out;
+  __device__ void operator()(long long q, long long at) const {
+    const int4* a = reinterpret_cast<const int4*>(h + q);
+    int4* b = reinterpret_cast<int4*>(out + at);
+    b[0] = a[0];
+    b[1] = a[1];
+  }
+};
+struct PutIndex {
+  int32_t* idx;
+  __device__ void operator()(long long q, long long at) const { idx[at] = (int32_t)q; }
+};
+
+cudaError_t compact_cells(const rpd_cell_header* pair_headers, long long n_pairs,
+                          int32_t* scan_tmp, rpd_cell_header* out, long long* n_out_dev,
+                          unsigned long long* status_hist, cudaStream_t st,
                           unsigned long long* n_uncert) {
-  int nb = (int)((n_pairs + 255) / 256);
-  if (n_pairs > 0) {
-    flag_cells_kernel<<<nb, 256, 0, st>>>(pair_headers, n_pairs, flag_tmp, status_hist, n_uncert);
-    note_launches(1);
-  }
-  cudaError_t err = scan_exclusive(flag_tmp, pos_tmp, n_pairs, scan_tmp, st);
-  if (err != cudaSuccess) return err;
-  gather_cells_kernel<<<nb > 0 ? nb : 1, 256, 0, st>>>(pair_headers, n_pairs, pos_tmp, out, n_out_dev);
-  note_launches(1);
-  return cudaGetLastError();
+  return keep_indices(CountCells{pair_headers, status_hist, n_uncert},
+                      HasStatus{pair_headers, kSuccess}, PutHeader{pair_headers, out}, n_pairs,
+                      scan_tmp, n_out_dev, st);
 }
 
-__global__ void flag_status_kernel(const rpd_cell_header* h, long long n, int status,
-                                   int32_t* flag) {
-  long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) flag[q] = h[q].status == status ? 1 : 0;
+cudaError_t select_pairs(const rpd_cell_header* h, long long n, int status, int32_t* scan_tmp,
+                         int32_t* idx_out, int32_t* count_out, cudaStream_t st) {
+  const HasStatus t{h, status};
+  return keep_indices(Plain<HasStatus>{t}, t, PutIndex{idx_out}, n, scan_tmp, count_out, st);
 }
 
-__global__ void scatter_index_kernel(const int32_t* flag, const int32_t* pos, long long n,
-                                     int32_t* idx) {
-  long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n && flag[q]) idx[pos[q]] = (int32_t)q;
+cudaError_t select_uncertified(const rpd_cell_header* h, long long n, int32_t* scan_tmp,
+                               int32_t* idx_out, int32_t* count_out, cudaStream_t st) {
+  const IsUncertified t{h};
+  return keep_indices(Plain<IsUncertified>{t}, t, PutIndex{idx_out}, n, scan_tmp, count_out, st);
 }
 
-cudaError_t select_pairs(const rpd_cell_header* h, long long n, int status, int32_t* flag_tmp,
-                         int32_t* pos_tmp, int32_t* scan_tmp, int32_t* idx_out,
-                         cudaStream_t st) {
-  int nb = (int)((n + 255) / 256);
-  if (n > 0) {
-    flag_status_kernel<<<nb, 256, 0, st>>>(h, n, status, flag_tmp);
-    note_launches(1);
-  }
-  cudaError_t err = scan_exclusive(flag_tmp, pos_tmp, n, scan_tmp, st);
-  if (err != cudaSuccess) return err;
-  if (n > 0) {
-    scatter_index_kernel<<<nb, 256, 0, st>>>(flag_tmp, pos_tmp, n, idx_out);
-    note_launches(1);
-  }
-  return cudaGetLastError();
-}
-
-__global__ void flag_uncert_kernel(const rpd_cell_header* h, long long n, int32_t* flag) {
-  long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) {
-    const rpd_cell_header hq = h[q];
-    flag[q] = (hq.status == kSuccess && (hq.flags & RPD_CELL_UNCERTIFIED)) ? 1 : 0;
-  }
-}
-
-cudaError_t select_uncertified(const rpd_cell_header* h, long long n, int32_t* flag_tmp,
-                               int32_t* pos_tmp, int32_t* scan_tmp, int32_t* idx_out,
-                               cudaStream_t st) {
-  int nb = (int)((n + 255) / 256);
-  if (n > 0) {
-    flag_uncert_kernel<<<nb, 256, 0, st>>>(h, n, flag_tmp);
-    note_launches(1);
-  }
-  cudaError_t err = scan_exclusive(flag_tmp, pos_tmp, n, scan_tmp, st);
-  if (err != cudaSuccess) return err;
-  if (n > 0) {
-    scatter_index_kernel<<<nb, 256, 0, st>>>(flag_tmp, pos_tmp, n, idx_out);
-    note_launches(1);
-  }
-  return cudaGetLastError();
-}
-
-__global__ void flag_need_kernel(const unsigned int* need, int n, int32_t* flag) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) flag[i] = need[i] != 0u ? 1 : 0;
-}
-
-cudaError_t select_sites(const unsigned int* site_need, int n, int32_t* flag_tmp,
-                         int32_t* pos_tmp, int32_t* scan_tmp, int32_t* idx_out, cudaStream_t st) {
-  int nb = (n + 255) / 256;
-  if (n > 0) {
-    flag_need_kernel<<<nb, 256, 0, st>>>(site_need, n, flag_tmp);
-    note_launches(1);
-  }
-  cudaError_t err = scan_exclusive(flag_tmp, pos_tmp, n, scan_tmp, st);
-  if (err != cudaSuccess) return err;
-  if (n > 0) {
-    scatter_index_kernel<<<nb, 256, 0, st>>>(flag_tmp, pos_tmp, n, idx_out);
-    note_launches(1);
-  }
-  return cudaGetLastError();
+cudaError_t select_sites(const unsigned int* site_need, int n, int32_t* scan_tmp,
+                         int32_t* idx_out, int32_t* count_out, cudaStream_t st) {
+  const IsNeeded t{site_need};
+  return keep_indices(Plain<IsNeeded>{t}, t, PutIndex{idx_out}, (long long)n, scan_tmp, count_out,
+                      st);
 }
 
 __global__ void assign_rows_kernel(const int32_t* sites, int n, int row0, long long off0,

@@ -41,35 +41,6 @@ namespace rpd {
 
 namespace {
 
-constexpr int kScan64 = 1024;
-
-__global__ void scan64_reduce_kernel(const int32_t* in, long long n, long long* sums) {
-  const long long i = (long long)blockIdx.x * kScan64 + threadIdx.x;
-  long long tot;
-  block_excl_scan<long long>(i < n ? in[i] : 0, &tot);
-  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
-}
-
-__global__ void scan64_blocksums_kernel(long long* sums, int nb) {
-  long long carry = 0;
-  for (int base = 0; base < nb; base += kScan64) {
-    const int i = base + threadIdx.x;
-    long long tot;
-    const long long ex = block_excl_scan<long long>(i < nb ? sums[i] : 0, &tot);
-    if (i < nb) sums[i] = ex + carry;
-    carry += tot;
-  }
-  if (threadIdx.x == 0) sums[nb] = carry;
-}
-
-__global__ void scan64_apply_kernel(const int32_t* in, long long n, const long long* sums, int nb,
-                                    long long* out) {
-  const long long i = (long long)blockIdx.x * kScan64 + threadIdx.x;
-  const long long ex = block_excl_scan<long long>(i < n ? in[i] : 0, nullptr);
-  if (i < n) out[i] = ex + sums[blockIdx.x];
-  if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = sums[nb];
-}
-
 __device__ __forceinline__ bool face_shown(int2 hp, const PolyParams& p) {
   return !p.boundary_only || hp.y != -1 || hp.x < p.max_sf_fid;
 }
@@ -274,17 +245,11 @@ cudaError_t bgeo_fill(const float* points, long long n_points, const long long* 
   return cudaGetLastError();
 }
 
-size_t scan64_temp(long long n) { return (size_t)((n + kScan64 - 1) / kScan64) + 1; }
+size_t scan64_temp(long long n) { return (size_t)((n + kScanTile - 1) / kScanTile) + 1; }
 
 cudaError_t scan64_exclusive(const int32_t* in, long long* out, long long n, long long* temp,
                              cudaStream_t st) {
-  const int nb = (int)((n + kScan64 - 1) / kScan64);
-  if (nb == 0) return cudaMemsetAsync(out, 0, sizeof(long long), st);
-  scan64_reduce_kernel<<<nb, kScan64, 0, st>>>(in, n, temp);
-  scan64_blocksums_kernel<<<1, kScan64, 0, st>>>(temp, nb);
-  scan64_apply_kernel<<<nb, kScan64, 0, st>>>(in, n, temp, nb, out);
-  note_launches(3);
-  return cudaGetLastError();
+  return scan_counts<long long>(in, out, n, temp, st);
 }
 
 cudaError_t poly_count(const PolyParams& p, cudaStream_t st) {
