@@ -288,7 +288,8 @@ void rpd_destroy(rpd_ctx* c) {
   c->s_cell_fill.release(); c->s_cell_items.release();
   c->t_cell_of.release(); c->t_cell_count.release(); c->t_cell_start.release();
   c->t_cell_fill.release(); c->t_cell_items.release();
-  c->centroid.release(); c->site_box.release(); c->site_planes.release();
+  c->centroid.release(); c->site_box.release(); c->site_box1.release(); c->site_planes.release();
+  c->t_cell_cent.release(); c->t_cell_xyz.release();
   c->site_nplanes.release(); c->pair_ntasks.release(); c->pair_taskoff.release(); c->scan_tmp.release();
   c->pair_buf.release(); c->tet_count.release(); c->tet_offsets.release();
   c->tet_fill.release(); c->pair_site.release(); c->pair_tet.release();
@@ -969,6 +970,9 @@ rpd_status rpd_compute(rpd_ctx* c, rpd_stats* stats) {
     const int32_t* box_list = knn ? c->nbr_dist.ptr : c->nbr.ptr;
     const int box0 = c->cfg.box_planes > 0 ? c->cfg.box_planes : kDefaultBoxPlanes;
     CK(c->site_box.ensure((size_t)n_site * 2), "alloc");
+    CK(c->site_box1.ensure((size_t)n_site * 2), "alloc");
+    CK(c->t_cell_cent.ensure((size_t)n_tet), "alloc");
+    CK(c->t_cell_xyz.ensure((size_t)n_tet * 3), "alloc");
     CK(c->site_planes.ensure((size_t)n_site * kBoxPlanes), "alloc");
     CK(c->site_nplanes.ensure((size_t)n_site), "alloc");
     CK(c->tet_count.ensure(n_tet), "alloc");
@@ -991,26 +995,32 @@ rpd_status rpd_compute(rpd_ctx* c, rpd_stats* stats) {
         CK(c->scan_tmp.ensure(scan_temp_ints(std::max<long long>(nc, n_tet)) + 16), "alloc");
         CK(grid_build_tets(c->centroid.ptr, n_tet, c->tet_class.ptr, cl, tg, c->t_cell_of.ptr,
                            c->t_cell_count.ptr, c->t_cell_start.ptr, c->t_cell_fill.ptr,
-                           c->t_cell_items.ptr, c->scan_tmp.ptr, st, c->t_cell_rmax.ptr), "tet grid");
+                           c->t_cell_items.ptr, c->scan_tmp.ptr, st, c->t_cell_rmax.ptr,
+                           c->tet_xyz.ptr, c->t_cell_cent.ptr, c->t_cell_xyz.ptr), "tet grid");
         // per-site boxes: every tet of this class that passes the rule has
         // its centroid in the site's cell pushed out by the class radius
-        const double R = c->class_radius[cl] * (1.0 + 1e-5) + 1e-6 * cs;
+        // (a second class of larger tets takes its regions from the first's
+        // clip); the nearest bisectors bound the common tets, and a looser
+        // region with few planes does for the few large ones
+        auto pushed = [&](int k) { return (float)(c->class_radius[k] * (1.0 + 1e-5) + 1e-6 * cs); };
+        const bool second = cl > 0 && c->class_count[0] > 0;
+        auto k_box = [&](int k) { return knn ? std::min(c->k, k == 0 ? box0 : std::min(box0, 12)) : c->k; };
         BoxParams bp;
         bp.site4f = c->site4f.ptr;
         bp.flags = c->flags.ptr;
         bp.site_base = 0;
         bp.nbr = box_list;
         bp.k = c->k;
-        // the nearest bisectors (distance-ordered GPU lists) for the common
-        // tets; the class of the largest tets has few tets, so a looser
-        // region costs little in the search and its box is cheap to clip
-        bp.k_box = knn ? std::min(c->k, cl == 0 ? box0 : std::min(box0, 12)) : c->k;
+        bp.k_box = k_box(cl);
         bp.n_site = n_site;
         bp.box_lo = make_float4((float)(c->mesh_lo[0] - margin), (float)(c->mesh_lo[1] - margin),
                                 (float)(c->mesh_lo[2] - margin), 0.f);
         bp.box_hi = make_float4((float)(c->mesh_hi[0] + margin), (float)(c->mesh_hi[1] + margin),
                                 (float)(c->mesh_hi[2] + margin), 0.f);
-        bp.offset_r = (float)R;
+        bp.offset_r = pushed(cl);
+        bp.offset_r1 = cl == 0 && c->class_count[1] > 0 ? pushed(1) : 0.f;
+        bp.k_box1 = k_box(1);
+        bp.site_box1 = c->site_box1.ptr;
         bp.offset_e = (float)(48.0 * u * (diag2 + std::fabs((double)c->w_max)));
         bp.coord_scale = (float)cs;
         bp.abs_margin = (float)margin;
@@ -1020,17 +1030,17 @@ rpd_status rpd_compute(rpd_ctx* c, rpd_stats* stats) {
         bp.counters = nullptr;
         int bw = 4;
         int bblocks = std::max(1, std::min((n_site + bw - 1) / bw, c->num_sms * box_blocks_per_sm(bw)));
-        CK(launch_site_box(bp, bblocks, bw, st), "site boxes");
+        if (!second) CK(launch_site_box(bp, bblocks, bw, st), "site boxes");
         PairParams pp;
         pp.vert3f = c->vert3f.ptr;
         pp.tets = c->tets.ptr;
-        pp.centroid = c->centroid.ptr;
-        pp.tet_xyz = c->tet_xyz.ptr;
         pp.tet_base = 0;
         pp.site_base = 0;
         pp.tg = tg;
         pp.tcell_start = c->t_cell_start.ptr;
         pp.tcell_items = c->t_cell_items.ptr;
+        pp.tcell_cent = c->t_cell_cent.ptr;
+        pp.tcell_xyz = c->t_cell_xyz.ptr;
         pp.tcell_rmax = c->t_cell_rmax.ptr;
         pp.site4f = c->site4f.ptr;
         pp.flags = c->flags.ptr;
@@ -1038,8 +1048,9 @@ rpd_status rpd_compute(rpd_ctx* c, rpd_stats* stats) {
         pp.rule_nbr = knn ? c->nbr_dist.ptr : nullptr;
         pp.k = c->k;
         pp.n_site = n_site;
-        pp.site_box = c->site_box.ptr;
+        pp.site_box = second ? c->site_box1.ptr : c->site_box.ptr;
         pp.offset_r = bp.offset_r;
+        pp.plane_grow = second ? pushed(cl) - pushed(0) : 0.f;
         pp.rule_keys = knn ? c->nbr_keys.ptr : nullptr;
         pp.accept_margin = (float)(16.0 * u * (cs + std::sqrt(diag2)));
         pp.accept_err = 1.01f * bp.offset_e;

@@ -45,6 +45,7 @@ struct FrontLane {
   DevBuf<int32_t> s_cell_count, s_cell_start, s_cell_fill, s_cell_items;
   DevBuf<int32_t> t_cell_of, t_cell_count, t_cell_start, t_cell_fill, t_cell_items;
   DevBuf<float> t_cell_rmax;
+  DevBuf<float4> t_cell_cent, t_cell_xyz;
   DevBuf<int32_t> scan_tmp, pair_ntasks, pair_taskoff;
   DevBuf<unsigned long long> work;  // the pair kernel's task counter
   std::vector<int> meshes;           // meshes of this lane
@@ -166,6 +167,7 @@ rpd_status upload(rpd_batch* b) {
   BCK(c->nbr_bound.ensure((size_t)n_site), "alloc");
   BCK(c->s_cell_of.ensure((size_t)n_site), "alloc");
   BCK(c->site_box.ensure((size_t)n_site * 2), "alloc");
+  BCK(c->site_box1.ensure((size_t)n_site * 2), "alloc");
   BCK(c->site_planes.ensure((size_t)n_site * kBoxPlanes), "alloc");
   BCK(c->site_nplanes.ensure((size_t)n_site), "alloc");
   BCK(c->centroid.ensure((size_t)n_tet), "alloc");
@@ -208,6 +210,8 @@ rpd_status upload(rpd_batch* b) {
     BCK(L.s_cell_items.ensure((size_t)max_site), "alloc");
     BCK(L.t_cell_of.ensure((size_t)max_tet), "alloc");
     BCK(L.t_cell_items.ensure((size_t)max_tet), "alloc");
+    BCK(L.t_cell_cent.ensure((size_t)max_tet), "alloc");
+    BCK(L.t_cell_xyz.ensure((size_t)max_tet * 3), "alloc");
     BCK(L.t_cell_count.ensure((size_t)max_tc), "alloc");
     BCK(L.t_cell_rmax.ensure((size_t)max_tc), "alloc");
     BCK(L.t_cell_start.ensure((size_t)max_tc + 1), "alloc");
@@ -281,22 +285,28 @@ rpd_status front_end(rpd_batch* b) {
       BCK(grid_build_tets(c->centroid.ptr + tb, m.n_tet, c->tet_class.ptr + tb, cl, tg,
                           L.t_cell_of.ptr, L.t_cell_count.ptr, L.t_cell_start.ptr,
                           L.t_cell_fill.ptr, L.t_cell_items.ptr, L.scan_tmp.ptr, ls,
-                          L.t_cell_rmax.ptr),
+                          L.t_cell_rmax.ptr, c->tet_xyz.ptr + 3ll * tb, L.t_cell_cent.ptr,
+                          L.t_cell_xyz.ptr),
           "tet grid");
-      const double R = m.class_radius[cl] * (1.0 + 1e-5) + 1e-6 * cs;
+      auto pushed = [&](int q) { return (float)(m.class_radius[q] * (1.0 + 1e-5) + 1e-6 * cs); };
+      const bool second = cl > 0 && m.class_count[0] > 0;
+      auto k_box = [&](int q) { return std::min(k, q == 0 ? box0 : std::min(box0, 12)); };
       BoxParams bp;
       bp.site4f = c->site4f.ptr;
       bp.flags = c->flags.ptr;
       bp.site_base = sb;
       bp.nbr = c->nbr_dist.ptr + (long long)sb * k;
       bp.k = k;
-      bp.k_box = std::min(k, cl == 0 ? box0 : std::min(box0, 12));
+      bp.k_box = k_box(cl);
       bp.n_site = m.n_site;
       bp.box_lo = make_float4((float)(m.mesh_lo[0] - margin), (float)(m.mesh_lo[1] - margin),
                               (float)(m.mesh_lo[2] - margin), 0.f);
       bp.box_hi = make_float4((float)(m.mesh_hi[0] + margin), (float)(m.mesh_hi[1] + margin),
                               (float)(m.mesh_hi[2] + margin), 0.f);
-      bp.offset_r = (float)R;
+      bp.offset_r = pushed(cl);
+      bp.offset_r1 = cl == 0 && m.class_count[1] > 0 ? pushed(1) : 0.f;
+      bp.k_box1 = k_box(1);
+      bp.site_box1 = c->site_box1.ptr + 2ll * sb;
       bp.offset_e = (float)(48.0 * u * (diag2 + std::fabs((double)m.w_max)));
       bp.coord_scale = (float)cs;
       bp.abs_margin = (float)margin;
@@ -306,17 +316,17 @@ rpd_status front_end(rpd_batch* b) {
       bp.counters = nullptr;
       const int bw = 4;
       const int bblocks = std::max(1, std::min((m.n_site + bw - 1) / bw, c->num_sms * box_blocks_per_sm(bw)));
-      BCK(launch_site_box(bp, bblocks, bw, ls), "site boxes");
+      if (!second) BCK(launch_site_box(bp, bblocks, bw, ls), "site boxes");
       PairParams pp;
       pp.vert3f = c->vert3f.ptr;
       pp.tets = c->tets.ptr + tb;
-      pp.centroid = c->centroid.ptr + tb;
-      pp.tet_xyz = c->tet_xyz.ptr + 3ll * tb;
       pp.tet_base = tb;
       pp.site_base = sb;
       pp.tg = tg;
       pp.tcell_start = L.t_cell_start.ptr;
       pp.tcell_items = L.t_cell_items.ptr;
+      pp.tcell_cent = L.t_cell_cent.ptr;
+      pp.tcell_xyz = L.t_cell_xyz.ptr;
       pp.tcell_rmax = L.t_cell_rmax.ptr;
       pp.site4f = c->site4f.ptr;
       pp.flags = c->flags.ptr;
@@ -324,9 +334,12 @@ rpd_status front_end(rpd_batch* b) {
       pp.rule_nbr = c->nbr_dist.ptr + (long long)sb * k;
       pp.k = k;
       pp.n_site = m.n_site;
-      pp.site_box = c->site_box.ptr + 2ll * sb;
+      pp.site_box = (second ? c->site_box1.ptr : c->site_box.ptr) + 2ll * sb;
       pp.offset_r = bp.offset_r;
-      pp.rule_keys = nullptr;  // (the rule checks every neighbour)
+      pp.plane_grow = second ? pushed(cl) - pushed(0) : 0.f;
+      pp.rule_keys = c->nbr_keys.ptr + (long long)sb * k;
+      pp.accept_margin = (float)(16.0 * u * (cs + std::sqrt(diag2)));
+      pp.accept_err = 1.01f * bp.offset_e;
       pp.site_planes = c->site_planes.ptr + (long long)sb * kBoxPlanes;
       pp.site_nplanes = c->site_nplanes.ptr + sb;
       pp.coord_scale = (float)cs;

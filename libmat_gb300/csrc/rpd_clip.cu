@@ -1011,127 +1011,184 @@ __global__ void __launch_bounds__(128, 6) site_box_kernel(BoxParams p) {
       if (lane == 0) {
         p.site_box[2 * i] = make_float4(1.f, 1.f, 1.f, 0.f);  // empty box
         p.site_box[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.offset_r1 > 0.f) {
+          p.site_box1[2 * i] = make_float4(1.f, 1.f, 1.f, 0.f);
+          p.site_box1[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         p.site_nplanes[i] = 0;
       }
       continue;
     }
     const float4 seed = p.site4f[p.site_base + i];
-    // box planes x>=lo, x<=hi, y>=lo, y<=hi, z>=lo, z<=hi
-    if (lane < 6) {
-      int ax = lane >> 1;
-      float4 pl = make_float4(0.f, 0.f, 0.f, 0.f);
-      float* q = reinterpret_cast<float*>(&pl);
-      if ((lane & 1) == 0) {
-        q[ax] = 1.f;
-        pl.w = -lo[ax];
-      } else {
-        q[ax] = -1.f;
-        pl.w = hi[ax];
+    // own: the second class's region by a clip of its own, because the first
+    // class's is empty
+    for (bool own = false;;) {
+      // box planes x>=lo, x<=hi, y>=lo, y<=hi, z>=lo, z<=hi
+      if (lane < 6) {
+        int ax = lane >> 1;
+        float4 pl = make_float4(0.f, 0.f, 0.f, 0.f);
+        float* q = reinterpret_cast<float*>(&pl);
+        if ((lane & 1) == 0) {
+          q[ax] = 1.f;
+          pl.w = -lo[ax];
+        } else {
+          q[ax] = -1.f;
+          pl.w = hi[ax];
+        }
+        c.pl[lane] = pl;
+      } else if (lane < 14) {
+        // corner (sx, sy, sz): planes X = sx, Y = 2 + sy, Z = 4 + sz, ordered
+        // (X, Z, Y) for even parity and (X, Y, Z) for odd parity: the eight
+        // dual triangles are then consistently oriented with the same sign as
+        // the tet's (det4x4 of the triangle's planes with (0,0,0,1) < 0), so
+        // "det > 0" means "outside" for both
+        int v = lane - 6;
+        int sx = v & 1, sy = (v >> 1) & 1, sz = (v >> 2) & 1;
+        uint8_t X = (uint8_t)sx, Y = (uint8_t)(2 + sy), Z = (uint8_t)(4 + sz);
+        c.ver[v] = ((sx + sy + sz) & 1) == 0 ? make_uchar4(X, Z, Y, 0) : make_uchar4(X, Y, Z, 0);
       }
-      c.pl[lane] = pl;
-    } else if (lane < 14) {
-      // corner (sx, sy, sz): planes X = sx, Y = 2 + sy, Z = 4 + sz, ordered
-      // (X, Z, Y) for even parity and (X, Y, Z) for odd parity: the eight
-      // dual triangles are then consistently oriented with the same sign as
-      // the tet's (det4x4 of the triangle's planes with (0,0,0,1) < 0), so
-      // "det > 0" means "outside" for both
-      int v = lane - 6;
-      int sx = v & 1, sy = (v >> 1) & 1, sz = (v >> 2) & 1;
-      uint8_t X = (uint8_t)sx, Y = (uint8_t)(2 + sy), Z = (uint8_t)(4 + sz);
-      c.ver[v] = ((sx + sy + sz) & 1) == 0 ? make_uchar4(X, Z, Y, 0) : make_uchar4(X, Y, Z, 0);
-    }
-    __syncwarp();
-    CellState s;
-    s.nb_v = 8;
-    s.nb_p = 6;
-    s.nb_e = 0;
-    s.status = kSuccess;
-    refresh_cofactors<RPD_PRED_FP32_FILTER, false>(c, 0, 8, lane, make_float3(0.f, 0.f, 0.f));
-    __syncwarp();
-    const float4* site4f = p.site4f;
-    const float R = p.offset_r, E = p.offset_e;
-    auto make_plane = [&](int j) {
-      float4 b = __ldg(site4f + j);
-      float4 e = bisector_f(seed, b);
-      float D = sqrtf(e.x * e.x + e.y * e.y + e.z * e.z);
-      // push the plane outwards by R plus the float error of the rule's
-      // power distances (E / 2D) plus a relative slack
-      float slack = 1e-5f * (fabsf(e.w) + D * p.coord_scale);
-      float d = e.w + R * D + 0.5f * E + slack;
-      if (!(D > 0.f) || !(d < 3.0e38f)) return make_float4(0.f, 0.f, 0.f, 1.f);  // no constraint
-      return make_float4(e.x, e.y, e.z, d);
-    };
-    // any subset of the planes gives a superset polytope; the nearest k_box
-    // bisectors bound the cell well and keep the box clip small
-    Cert nocert;
-    nocert.keys = nullptr;
-    nocert.certified = false;
-    clip_list<RPD_PRED_FP32_FILTER, false, false>(c, s, p.nbr + (long long)i * p.k, p.k_box,
-                                                  p.site_base + i,
-                                                  make_plane, lane, pc, nocert);
-    float bl[3], bh[3];
-    if (s.status == kSuccess) {
-      bl[0] = bl[1] = bl[2] = 3.0e38f;
-      bh[0] = bh[1] = bh[2] = -3.0e38f;
-      for (int v = lane; v < s.nb_v; v += 32) {
-        uchar4 tr = c.ver[v];
-        float xl[3], xh[3];
-        vertex_of_float_planes(c.pl[tr.x], c.pl[tr.y], c.pl[tr.z], xl, xh);
-        for (int k = 0; k < 3; ++k) {
-          if (!(xl[k] == xl[k]) || !(xh[k] == xh[k])) {  // degenerate vertex
-            xl[k] = lo[k];
-            xh[k] = hi[k];
+      __syncwarp();
+      CellState s;
+      s.nb_v = 8;
+      s.nb_p = 6;
+      s.nb_e = 0;
+      s.status = kSuccess;
+      refresh_cofactors<RPD_PRED_FP32_FILTER, false>(c, 0, 8, lane, make_float3(0.f, 0.f, 0.f));
+      __syncwarp();
+      const float4* site4f = p.site4f;
+      const float R = own ? p.offset_r1 : p.offset_r, E = p.offset_e;
+      auto make_plane = [&](int j) {
+        float4 b = __ldg(site4f + j);
+        float4 e = bisector_f(seed, b);
+        float D = sqrtf(e.x * e.x + e.y * e.y + e.z * e.z);
+        // push the plane outwards by R plus the float error of the rule's
+        // power distances (E / 2D) plus a relative slack
+        float slack = 1e-5f * (fabsf(e.w) + D * p.coord_scale);
+        float d = e.w + R * D + 0.5f * E + slack;
+        if (!(D > 0.f) || !(d < 3.0e38f)) return make_float4(0.f, 0.f, 0.f, 1.f);  // no constraint
+        return make_float4(e.x, e.y, e.z, d);
+      };
+      // any subset of the planes gives a superset polytope; the nearest k_box
+      // bisectors bound the cell well and keep the box clip small
+      Cert nocert;
+      nocert.keys = nullptr;
+      nocert.certified = false;
+      clip_list<RPD_PRED_FP32_FILTER, false, false>(c, s, p.nbr + (long long)i * p.k,
+                                                    own ? p.k_box1 : p.k_box, p.site_base + i,
+                                                    make_plane, lane, pc, nocert);
+      float bl[3], bh[3];
+      if (s.status == kSuccess) {
+        bl[0] = bl[1] = bl[2] = 3.0e38f;
+        bh[0] = bh[1] = bh[2] = -3.0e38f;
+        for (int v = lane; v < s.nb_v; v += 32) {
+          uchar4 tr = c.ver[v];
+          float xl[3], xh[3];
+          vertex_of_float_planes(c.pl[tr.x], c.pl[tr.y], c.pl[tr.z], xl, xh);
+          for (int k = 0; k < 3; ++k) {
+            if (!(xl[k] == xl[k]) || !(xh[k] == xh[k])) {  // degenerate vertex
+              xl[k] = lo[k];
+              xh[k] = hi[k];
+            }
+            bl[k] = fminf(bl[k], xl[k]);
+            bh[k] = fmaxf(bh[k], xh[k]);
           }
-          bl[k] = fminf(bl[k], xl[k]);
-          bh[k] = fmaxf(bh[k], xh[k]);
         }
-      }
-      for (int o = 16; o > 0; o >>= 1)
+        for (int o = 16; o > 0; o >>= 1)
+          for (int k = 0; k < 3; ++k) {
+            bl[k] = fminf(bl[k], __shfl_xor_sync(0xffffffffu, bl[k], o));
+            bh[k] = fmaxf(bh[k], __shfl_xor_sync(0xffffffffu, bh[k], o));
+          }
         for (int k = 0; k < 3; ++k) {
-          bl[k] = fminf(bl[k], __shfl_xor_sync(0xffffffffu, bl[k], o));
-          bh[k] = fmaxf(bh[k], __shfl_xor_sync(0xffffffffu, bh[k], o));
+          float m = 1e-3f * (bh[k] - bl[k]) + p.abs_margin;
+          bl[k] = fmaxf(bl[k] - m, lo[k]);
+          bh[k] = fminf(bh[k] + m, hi[k]);
         }
-      for (int k = 0; k < 3; ++k) {
-        float m = 1e-3f * (bh[k] - bl[k]) + p.abs_margin;
-        bl[k] = fmaxf(bl[k] - m, lo[k]);
-        bh[k] = fminf(bh[k] + m, hi[k]);
+      } else if (s.status == kNoIntersection) {
+        bl[0] = bl[1] = bl[2] = 1.f;
+        bh[0] = bh[1] = bh[2] = 0.f;
+      } else {
+        for (int k = 0; k < 3; ++k) {
+          bl[k] = lo[k];
+          bh[k] = hi[k];
+        }
       }
-    } else if (s.status == kNoIntersection) {
-      bl[0] = bl[1] = bl[2] = 1.f;
-      bh[0] = bh[1] = bh[2] = 0.f;
-    } else {
-      for (int k = 0; k < 3; ++k) {
-        bl[k] = lo[k];
-        bh[k] = hi[k];
+      const bool empty = s.status == kNoIntersection;
+      if (lane == 0) {
+        float4* box = own ? p.site_box1 : p.site_box;
+        box[2 * i] = make_float4(bl[0], bl[1], bl[2], own ? 1.f : 0.f);
+        box[2 * i + 1] = make_float4(bh[0], bh[1], bh[2], 0.f);
       }
+      if (empty && !own && p.offset_r1 > 0.f) {
+        __syncwarp();
+        own = true;
+        continue;
+      }
+      // the planes that bound the grown cell (referenced by a vertex): the pair
+      // search tests grid cells and tet centroids against them
+      int npl = 0;
+      unsigned long long bounding = 0ull;
+      if (s.status == kSuccess) {
+        unsigned long long m = 0ull;
+        for (int v = lane; v < s.nb_v; v += 32) {
+          uchar4 tr = c.ver[v];
+          m |= (1ull << tr.x) | (1ull << tr.y) | (1ull << tr.z);
+        }
+        const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)m);
+        const uint32_t hi = __reduce_or_sync(0xffffffffu, (uint32_t)(m >> 32));
+        const unsigned long long act = ((unsigned long long)hi << 32) | lo;
+        bounding = act;
+        // any subset of them bounds a superset of the grown cell: beyond the
+        // storage, the first kBoxPlanes are kept
+        npl = min(__popcll(act), kBoxPlanes);
+        for (int q = lane; q < s.nb_p; q += 32) {
+          const int rank = __popcll(act & ((1ull << q) - 1ull));
+          if (((act >> q) & 1ull) && rank < kBoxPlanes)
+            p.site_planes[(long long)i * kBoxPlanes + rank] = c.pl[q];
+        }
+      }
+      if (lane == 0) p.site_nplanes[i] = npl;
+      if (!own && p.offset_r1 > 0.f) {
+        // The larger class's region from this one: pushing every bounding plane
+        // out by delta stays inside the polytope scaled about the seed by
+        // lambda = 1 + delta / h, h the seed's least distance to those planes
+        // (a point x of it has x / lambda on their inner side, since (h_m +
+        // delta) / lambda <= h_m).  It saves that class's clip, 0.63 ms of the
+        // 1M-tet workload for 0.5 % of its tets.  A seed outside or close to a
+        // plane gets the whole region, whose grid cells the planes then cull.
+        const float delta = (p.offset_r1 - p.offset_r) * (1.0f + 1e-4f);
+        float h = INFINITY;
+        if (s.status == kSuccess) {
+          for (int q = lane; q < s.nb_p; q += 32)
+            if ((bounding >> q) & 1ull) {
+              const float4 e = c.pl[q];
+              const float tol = 4e-6f * ((fabsf(e.x) + fabsf(e.y) + fabsf(e.z)) * p.coord_scale +
+                                         fabsf(e.w));
+              const float v = e.x * seed.x + e.y * seed.y + e.z * seed.z + e.w - tol;
+              h = fminf(h, v / sqrtf(e.x * e.x + e.y * e.y + e.z * e.z));
+            }
+          for (int o = 16; o > 0; o >>= 1) h = fminf(h, __shfl_xor_sync(0xffffffffu, h, o));
+        }
+        if (lane == 0) {
+          const bool scaled = s.status == kSuccess && h > 1e-2f * delta && h < INFINITY;
+          const float lam = scaled ? 1.0f + delta / h * (1.0f + 1e-4f) : 0.f;
+          const float sd[3] = {seed.x, seed.y, seed.z};
+          float l1[3], h1[3];
+          for (int k = 0; k < 3; ++k) {
+            l1[k] = lo[k];
+            h1[k] = hi[k];
+            if (scaled) {
+              const float m = 1e-3f * lam * (bh[k] - bl[k]) + p.abs_margin;
+              l1[k] = fmaxf(sd[k] - lam * (sd[k] - bl[k]) - m, lo[k]);
+              h1[k] = fminf(sd[k] + lam * (bh[k] - sd[k]) + m, hi[k]);
+            }
+          }
+          p.site_box1[2 * i] = make_float4(l1[0], l1[1], l1[2], 0.f);
+          p.site_box1[2 * i + 1] = make_float4(h1[0], h1[1], h1[2], 0.f);
+        }
+      }
+      __syncwarp();
+      break;
     }
-    if (lane == 0) {
-      p.site_box[2 * i] = make_float4(bl[0], bl[1], bl[2], (float)s.status);
-      p.site_box[2 * i + 1] = make_float4(bh[0], bh[1], bh[2], 0.f);
-    }
-    // the planes that bound the grown cell (referenced by a vertex): the pair
-    // search tests grid cells and tet centroids against them
-    int npl = 0;
-    if (s.status == kSuccess) {
-      unsigned long long m = 0ull;
-      for (int v = lane; v < s.nb_v; v += 32) {
-        uchar4 tr = c.ver[v];
-        m |= (1ull << tr.x) | (1ull << tr.y) | (1ull << tr.z);
-      }
-      uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)m);
-      uint32_t hi = __reduce_or_sync(0xffffffffu, (uint32_t)(m >> 32));
-      unsigned long long act = ((unsigned long long)hi << 32) | lo;
-      // any subset of them bounds a superset of the grown cell: beyond the
-      // storage, the first kBoxPlanes are kept
-      npl = min(__popcll(act), kBoxPlanes);
-      for (int q = lane; q < s.nb_p; q += 32) {
-        const int rank = __popcll(act & ((1ull << q) - 1ull));
-        if (((act >> q) & 1ull) && rank < kBoxPlanes)
-          p.site_planes[(long long)i * kBoxPlanes + rank] = c.pl[q];
-      }
-    }
-    if (lane == 0) p.site_nplanes[i] = npl;
-    __syncwarp();
   }
   for (int o = 16; o > 0; o >>= 1) {
     pc.pred += __shfl_xor_sync(0xffffffffu, pc.pred, o);

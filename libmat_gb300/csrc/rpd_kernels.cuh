@@ -135,6 +135,12 @@ struct BoxParams {
   float coord_scale;      // largest coordinate magnitude
   float abs_margin;
   float4* site_box;       // n_site x 2: (lo, status), (hi, 0)
+  // the regions of a second class of larger tets, of radius offset_r1 (0:
+  // none): site_box1 as site_box, its status 1 where the stored planes are
+  // that class's own (the first class's region was empty)
+  float offset_r1;
+  int k_box1;
+  float4* site_box1;
   float4* site_planes;    // n_site x kBoxPlanes: planes of the grown cell
   int32_t* site_nplanes;  // n_site: count (0 = use the box only)
   unsigned long long* counters;
@@ -181,7 +187,7 @@ cudaError_t scan_exclusive(const int32_t* in, int32_t* out, long long n, int32_t
                            cudaStream_t st);
 
 // bins points into grid cells: cell_of[n], cell_start[n_cells + 1],
-// cell_items[n] (ascending item id within a cell)
+// cell_items[n] (in no order within a cell)
 cudaError_t grid_build_sites(const float4* pts, int n, const Grid& g, int32_t* cell_of,
                              int32_t* cell_count, int32_t* cell_start, int32_t* cell_fill,
                              int32_t* cell_items, int32_t* scan_tmp, cudaStream_t st);
@@ -191,11 +197,13 @@ cudaError_t tet_centroids(const float* vert3f, const int4* tets, int n_tet, floa
                           cudaStream_t st, float4* tet_xyz = nullptr,
                           const int32_t* v_adjs = nullptr, uchar4* tet_vadj = nullptr);
 // bins the tets of radius class `want` (all tets when cls is null) by centroid;
-// cell_rmax (optional) gets the largest tet radius (centroid.w) of each cell
+// cell_rmax (optional) gets the largest tet radius (centroid.w) of each cell,
+// cent_out and xyz_out the items' centroids and packed vertices in item order
 cudaError_t grid_build_tets(const float4* centroid, int n_tet, const uint8_t* cls, int want,
                             const Grid& g, int32_t* cell_of, int32_t* cell_count,
                             int32_t* cell_start, int32_t* cell_fill, int32_t* cell_items,
-                            int32_t* scan_tmp, cudaStream_t st, float* cell_rmax = nullptr);
+                            int32_t* scan_tmp, cudaStream_t st, float* cell_rmax,
+                            const float4* tet_xyz, float4* cent_out, float4* xyz_out);
 
 // k smallest power-bisector distances per site (ties by id); lists in
 // distance order or sorted by id
@@ -243,13 +251,13 @@ cudaError_t launch_knn(const KnnArgs& a, cudaStream_t st);
 struct PairParams {
   const float* vert3f;     // all vertices (tets hold global vertex ids)
   const int4* tets;        // this mesh's tets
-  const float4* centroid;  // this mesh's tets
-  const float4* tet_xyz;   // this mesh's tets: vertices packed in 3 float4
   int tet_base;            // index of this mesh's first tet among all tets
   int site_base;
   Grid tg;
   const int32_t* tcell_start;
   const int32_t* tcell_items;
+  const float4* tcell_cent;  // the items' centroids (w = radius) and packed
+  const float4* tcell_xyz;   // vertices (3 float4), in the order of the items
   const float* tcell_rmax;  // largest tet radius of each tet-grid cell (may be null)
   const float4* site4f;   // all sites
   const uint32_t* flags;  // all sites
@@ -270,6 +278,10 @@ struct PairParams {
   // tet radius, rounded up): each centroid test takes back what its own
   // tet's radius does not need
   float offset_r;
+  // the stored planes are those of a class of smaller tets: push them out by
+  // this much more (0: they are this class's), except where site_box says
+  // that they are this class's own
+  float plane_grow;
   // keys of the rule's (distance-ordered) lists, or null; with them a tet
   // whose nearest vertex lies within the key of neighbour r (less the
   // margins) passes the rule for r and every later neighbour at once
