@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
                        0.5f * (hi.z - lo.z) + slack);
     // a sliver's vertex whose place is hardly known would send every test of
     // it to the filter, one lane at a time
-    if (!(em < 0.0625f * span)) out = kBack;
+    if (!(em < 0.25f * span)) out = kBack;
     return outside;
   };
 
