@@ -282,6 +282,7 @@ struct PairParams {
   // this much more (0: they are this class's), except where site_box says
   // that they are this class's own
   float plane_grow;
+  int task_cells;  // grid cells of a task (set by launch_pairs)
   // keys of the rule's (distance-ordered) lists, or null; with them a tet
   // whose nearest vertex lies within the key of neighbour r (less the
   // margins) passes the rule for r and every later neighbour at once
@@ -290,7 +291,7 @@ struct PairParams {
   float accept_err;     // bound on the float error of pd_m(v) - pd_i(v)
 };
 // n_tasks, task_off: n_site and n_site + 1 ints; work: one counter
-cudaError_t launch_pairs(const PairParams& p, int32_t* n_tasks, int32_t* task_off,
+cudaError_t launch_pairs(PairParams p, int32_t* n_tasks, int32_t* task_off,
                          int32_t* scan_tmp, unsigned long long* work, int num_sms,
                          cudaStream_t st);
 

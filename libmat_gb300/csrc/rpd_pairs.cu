@@ -505,15 +505,23 @@ __device__ __forceinline__ CellRange site_cells(const PairParams& p, int i) {
   return r;
 }
 
-constexpr int kPairTaskCells = 512;
+// grid cells of a task: a warp works through a task alone, and one whose tets
+// all pass takes about 5 us a cell, so few sites need short tasks for the
+// other warps to help; every task stages its site's planes and list, so many
+// sites want long ones.  Pair stage (ms) with 16 / 32 / 64 / 128 / 256 / 512
+// cells: 92 sites 0.17 / 0.18 / 0.20 / 0.23 / 0.24 / 0.24, 10k sites 1.43 / 1.18 /
+// 1.20 / 1.28 / 1.62 / 1.93, 50k sites - / 5.59 / 4.89 / 4.59 / 4.59 / 5.01.
+int pair_task_cells(int n_site) {
+  return n_site <= 512 ? 16 : (n_site <= 4096 ? 32 : (n_site <= 16384 ? 64 : 128));
+}
 
-// tasks per site: its box's grid cells in chunks of kPairTaskCells
+// tasks per site: its box's grid cells in chunks of task_cells
 __global__ void pair_tasks_kernel(PairParams p, int32_t* n_tasks) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.n_site) return;
   CellRange r = site_cells(p, i);
   long long n = (long long)r.sx * r.sy * r.sz;
-  n_tasks[i] = (int)((n + kPairTaskCells - 1) / kPairTaskCells);
+  n_tasks[i] = (int)((n + p.task_cells - 1) / p.task_cells);
 }
 
 // The tets' centroids and vertices are read in the order of the grid's items
@@ -560,8 +568,8 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
     const int chunk = (int)(task - task_off[i]);
     const CellRange cr = site_cells(p, i);
     const int n_all = cr.sx * cr.sy * cr.sz;
-    const int c_begin = chunk * kPairTaskCells;
-    const int n_iter = min(kPairTaskCells, n_all - c_begin);
+    const int c_begin = chunk * p.task_cells;
+    const int n_iter = min(p.task_cells, n_all - c_begin);
     const float4 blo = p.site_box[2 * i], bhi = p.site_box[2 * i + 1];
     // planes of the site's grown cell, each loosened by its own float
     // evaluation error so that the tests below never reject a centroid the
@@ -851,10 +859,11 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
   }
 }
 
-cudaError_t launch_pairs(const PairParams& p, int32_t* n_tasks, int32_t* task_off,
+cudaError_t launch_pairs(PairParams p, int32_t* n_tasks, int32_t* task_off,
                          int32_t* scan_tmp, unsigned long long* work, int num_sms,
                          cudaStream_t st) {
   if (p.n_site <= 0) return cudaSuccess;
+  p.task_cells = pair_task_cells(p.n_site);
   pair_tasks_kernel<<<(p.n_site + 255) / 256, 256, 0, st>>>(p, n_tasks);
   note_launches(1);
   cudaError_t err = scan_exclusive(n_tasks, task_off, p.n_site, scan_tmp, st);
