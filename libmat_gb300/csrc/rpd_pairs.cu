@@ -234,6 +234,9 @@ constexpr int kKnnLongBuf = 8192;  // long lists (k > kKnnBuf - 64): 64 KB, one 
 // times the warps measured the same)
 constexpr int kKnnSmallBuf = 512;
 constexpr int kKnnSmallWarps = 8;
+// blocks that must fit an SM: 64 registers (the sort of 512 entries holds 32);
+// 2 / 3 / 4 / 5 blocks take 1.49 / 1.12 / 1.05 / 1.16 ms there
+constexpr int kKnnSmallBlocks = 4;
 
 __device__ __forceinline__ uint32_t order_key(float f) {
   uint32_t u = __float_as_uint(f);
@@ -274,6 +277,77 @@ __device__ void warp_bitonic_sort(unsigned long long* buf, int n, int lane) {
   }
 }
 
+// the same for 32 PER entries in registers, of which the first `keep` come
+// back: lane l holds elements PER l .. PER l + PER - 1 of the network, so its
+// strides below PER need no exchange between lanes.  (Every exchange of the
+// sort above goes through shared memory: 512 entries take about 6,700 warp
+// instructions there and 3,400 here.)  The entries are read as they lie (a
+// sort may start from any order) and only the kept ones are written back.
+template <int PER>
+__device__ __forceinline__ void warp_register_sort(unsigned long long* buf, int lane, int keep) {
+  unsigned long long v[PER];
+#pragma unroll
+  for (int r = 0; r < PER; ++r) v[r] = buf[32 * r + lane];
+  auto exchange = [&](int r, int j, bool up) {
+    const unsigned long long a = v[r], b = v[r + j];
+    const bool swap = (a > b) == up;
+    v[r] = swap ? b : a;
+    v[r + j] = swap ? a : b;
+  };
+  // levels within a lane
+#pragma unroll
+  for (int k = 2; k < PER; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int r = 0; r < PER; ++r)
+        if ((r & j) == 0) exchange(r, j, (r & k) == 0);
+  // levels across lanes
+  for (int k = PER > 1 ? PER : 2; k <= 32 * PER; k <<= 1) {
+    const bool up = ((lane * PER) & k) == 0;
+    for (int j = k >> 1; j >= PER; j >>= 1) {
+      const int lj = j / PER;
+      const bool take_max = ((lane & lj) != 0) == up;
+#pragma unroll
+      for (int r = 0; r < PER; ++r) {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, v[r], lj);
+        v[r] = (o > v[r]) == take_max ? o : v[r];
+      }
+    }
+#pragma unroll
+    for (int j = PER >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int r = 0; r < PER; ++r)
+        if ((r & j) == 0) exchange(r, j, up);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < PER; ++r)
+    if (PER * lane + r < keep) buf[PER * lane + r] = v[r];
+  __syncwarp();
+}
+
+// buf[0..n) sorted, n a power of two and at least 32; only the first `keep`
+// entries are kept.  MAX: the largest n
+template <int MAX>
+__device__ __forceinline__ void warp_sort(unsigned long long* buf, int n, int lane, int keep) {
+  if (n <= 64) {
+    if (n < 64) buf[32 + lane] = ~0ull;
+    __syncwarp();
+    warp_register_sort<2>(buf, lane, keep);
+  } else if (n == 128) {
+    warp_register_sort<4>(buf, lane, keep);
+  } else if (n == 256) {
+    warp_register_sort<8>(buf, lane, keep);
+  } else if (n == 512) {
+    warp_register_sort<16>(buf, lane, keep);
+  } else if (MAX >= 1024 && n == 1024) {
+    warp_register_sort<32>(buf, lane, keep);
+  } else {
+    warp_bitonic_sort(buf, n, lane);
+  }
+}
+
 __device__ __forceinline__ int next_pow2(int x) {
   int p = 32;
   while (p < x) p <<= 1;
@@ -286,9 +360,15 @@ __device__ __forceinline__ int next_pow2(int x) {
 // searched until every site outside has a key above the k-th kept one (or
 // above B): keys of sites at distance >= D are >= (D^2 + w_i - w_max)/(2D).
 // Candidates collect in a per-warp buffer of BUF entries (key bits | id,
-// 64-bit) that is sorted and cut to k whenever it fills.
+// 64-bit) that is sorted and cut to k when it fills, and at the end of a ring
+// only where the k-th key may end the search.  Sorting bounds it: with a sort
+// after every ring, through shared memory, base lists of 128 for 50k sites took
+// 1.61 ms and the longer lists of 2.7k of them 0.51 ms; with the sorts that are
+// needed, in registers, and rings enumerated as shells 1.05 and 0.25 ms (200k
+// tets: 0.31 and 0.36 -> 0.18 and 0.10 ms).
 template <int BUF, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) knn_kernel(KnnArgs a) {
+__global__ void __launch_bounds__(WARPS * 32, WARPS == kKnnSmallWarps ? kKnnSmallBlocks : 1)
+    knn_kernel(KnnArgs a) {
   extern __shared__ __align__(16) unsigned long long knn_smem[];
   __shared__ int scnt[WARPS];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -314,18 +394,45 @@ __global__ void __launch_bounds__(WARPS * 32) knn_kernel(KnnArgs a) {
   if (lane == 0) scnt[wid] = 0;
   __syncwarp();
   unsigned long long kth = ~0ull;  // packed k-th best so far (after a sort)
-  int done = 0;
+  bool done = false;
+  bool sorted = true;  // the buffer holds the best of what was seen, in order
+  // sorts the cnt entries and keeps the best k
+  auto sort_cut = [&](int cnt) {
+    const int n = next_pow2(max(cnt, 1));
+    for (int q = cnt + lane; q < n; q += 32) buf[q] = ~0ull;
+    __syncwarp();
+    warp_sort<BUF>(buf, n, lane, k);
+    sorted = true;
+    if (cnt >= k) kth = buf[k - 1];
+    return min(cnt, k);
+  };
   for (int r = 0; r <= rmax && !done; ++r) {
+    // the cells at distance r (in cells): the two faces z = -r, r, then the
+    // four sides of each layer between them, 2 r cells a side
     const int side = 2 * r + 1;
-    const int n_cube = side * side * side;
+    const int n_face = side * side;
+    const int n_shell = r == 0 ? 1 : 2 * n_face + (side - 2) * 8 * r;
     auto cell_at = [&](int idx) -> int {
-      int dx = idx % side - r, dy = (idx / side) % side - r, dz = idx / (side * side) - r;
-      if (max(max(abs(dx), abs(dy)), abs(dz)) != r) return -1;
-      int x = cx + dx, y = cy + dy, z = cz + dz;
+      int dx, dy, dz;
+      if (idx < 2 * n_face) {
+        dz = idx < n_face ? -r : r;
+        const int q = idx < n_face ? idx : idx - n_face;
+        dy = q / side - r;
+        dx = q % side - r;
+      } else {
+        const int q = idx - 2 * n_face;
+        dz = q / (8 * r) - r + 1;
+        const int e = q % (8 * r);
+        const int t = e % (2 * r) - r;  // -r .. r - 1
+        const int edge = e / (2 * r);
+        dx = edge == 0 ? t : (edge == 1 ? r : (edge == 2 ? -t : -r));
+        dy = edge == 0 ? -r : (edge == 1 ? t : (edge == 2 ? r : -t));
+      }
+      const int x = cx + dx, y = cy + dy, z = cz + dz;
       if (x < 0 || y < 0 || z < 0 || x >= g.nx || y >= g.ny || z >= g.nz) return -1;
       return x + g.nx * (y + g.ny * z);
     };
-    for_items(n_cube, cell_at, a.cell_start, lane, [&](int at, bool valid) {
+    for_items(n_shell, cell_at, a.cell_start, lane, [&](int at, bool valid) {
       const int j = valid ? a.cell_items[at] : -1;
       bool take = false;
       unsigned long long packed = 0;
@@ -339,36 +446,40 @@ __global__ void __launch_bounds__(WARPS * 32) knn_kernel(KnnArgs a) {
       if (take) buf[base + __popc(m & ((1u << lane) - 1u))] = packed;
       __syncwarp();
       int cnt = base + __popc(m);
-      if (cnt > BUF - 32) {
-        // sort and keep the best k
-        for (int q = cnt + lane; q < BUF; q += 32) buf[q] = ~0ull;
-        __syncwarp();
-        warp_bitonic_sort(buf, BUF, lane);
-        cnt = min(cnt, k);
-        if (cnt >= k) kth = buf[k - 1];
-      }
+      if (m) sorted = false;
+      if (cnt > BUF - 32) cnt = sort_cut(cnt);
       if (lane == 0) scnt[wid] = cnt;
       __syncwarp();
     });
+    // done once no site outside the searched block can have a key of T or
+    // less: keys there are >= f(D) with D >= r * cell, f(D) = (D^2 + wi -
+    // wmax) / (2D) increasing in D
+    auto reached = [&](float T) {
+      const float D = (float)r * g.cell;
+      if (!(D > 0.f && T < INFINITY)) return false;
+      const float lb = (D * D + si.w - a.w_max) / (2.f * D);
+      return T < lb - 1e-4f * (fabsf(lb) + D);
+    };
+    // fewer than k so far: every key up to B is still wanted.  Else the k-th
+    // key of the last sort bounds the wanted ones, and only a search that it
+    // does not end sorts again for a smaller one
     int cnt = scnt[wid];
-    int n = next_pow2(max(cnt, 1));
-    for (int q = cnt + lane; q < n; q += 32) buf[q] = ~0ull;
+    if (cnt < k) {
+      done = reached(B);
+    } else {
+      done = kth != ~0ull && reached(fminf(B, key_value((uint32_t)(kth >> 32))));
+      if (!done && !sorted) {
+        cnt = sort_cut(cnt);
+        if (lane == 0) scnt[wid] = cnt;
+        done = reached(fminf(B, key_value((uint32_t)(kth >> 32))));
+      }
+    }
     __syncwarp();
-    warp_bitonic_sort(buf, n, lane);
-    cnt = min(cnt, k);
-    if (lane == 0) scnt[wid] = cnt;
-    float T = B;  // keys above T are not wanted
-    if (cnt >= k) {
-      kth = buf[k - 1];
-      T = fminf(T, key_value((uint32_t)(kth >> 32)));
-    }
-    // keys of sites outside the searched block are >= f(D) with
-    // D >= r * cell, f(D) = (D^2 + wi - wmax) / (2D) increasing in D
-    float D = (float)r * g.cell;
-    if (D > 0.f && T < INFINITY) {
-      float lb = (D * D + si.w - a.w_max) / (2.f * D);
-      if (T < lb - 1e-4f * (fabsf(lb) + D)) done = 1;
-    }
+  }
+  if (!sorted) {
+    const int c = sort_cut(scnt[wid]);
+    __syncwarp();
+    if (lane == 0) scnt[wid] = c;
     __syncwarp();
   }
   int cnt = scnt[wid];
@@ -398,7 +509,7 @@ __global__ void __launch_bounds__(WARPS * 32) knn_kernel(KnnArgs a) {
       buf[q] = v;
     }
     __syncwarp();
-    warp_bitonic_sort(buf, n, lane);
+    warp_sort<BUF>(buf, n, lane, k);
     for (int q = lane; q < k; q += 32)
       a.nbr[rb + q] = q < cnt ? (int32_t)buf[q] + a.id_offset : -1;
   }
