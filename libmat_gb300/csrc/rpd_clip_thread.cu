@@ -115,7 +115,7 @@ __device__ __noinline__ bool slow_conflict(float4 p1, float4 p2, float4 p3, floa
   const int s = filter_sign(K, M, e);
   if (s != 0) return s > 0;
   ++*esc;
-  if (PRED == RPD_PRED_EXACT) return exact_conflict(p1, p2, p3, e, exact);
+  if (PRED == RPD_PRED_EXACT) return exact_conflict(p1, p2, p3, e, M, exact);
   return det4x4_ref(p1, p2, p3, e) > 0.0;
 }
 

@@ -98,3 +98,26 @@ def test_user_lists_with_holes_duplicates_and_unflagged_sites():
     b, hb, (_, pb), _ = run(cfg, adj, rpd.PRED_FP32_FILTER, nbr=nbr)
     assert b.n_pairs == a.n_pairs >= MIN_PAIRS
     assert same_records(ha, pa, hb, pb)
+
+
+@pytest.mark.parametrize("n,m", [(14, 7), (16, 8)])
+def test_exact_signs_equal_the_oracle(n, m):
+    """Lattices whose coordinates are (m = 8) and are not (m = 7) short binary
+    fractions: determinants that vanish exactly, and ones that only nearly do."""
+    from oracle import oracle as O
+
+    cfg = W.config_lattice(n=n, m=m)
+    adj = rpd.mesh_adjacency(cfg["vert3d"].shape[0], cfg["tets"])
+    with rpd.RPD(predicate_mode=rpd.PRED_EXACT, knn_k=40, exact_lists=False) as r:
+        r.set_mesh(cfg["vert3d"], cfg["tets"], adj["v_adjs"], adj["e_adj6"], adj["f_adjs"],
+                   adj["f_ids"])
+        r.set_sites(cfg["sites"], cfg["flags"])
+        st = r.compute()
+        nbr = r.neighbor_lists(len(cfg["sites"]))
+        offs, ps = r.pairs(len(cfg["tets"]))
+        ph, p = r.pair_headers(), r.cells()[1]
+    assert st.n_pairs >= MIN_PAIRS and st.n_fp64_uncertain > 0
+    mesh = dict(vert3d=cfg["vert3d"], tets=cfg["tets"],
+                **{k: adj[k] for k in ("v_adjs", "e_adj6", "f_adjs", "f_ids")})
+    oh, op, _ = O.clip_cells(mesh, cfg["sites"], nbr, offs, ps, pred_mode=2)
+    assert same_records(ph, p, oh, op)
