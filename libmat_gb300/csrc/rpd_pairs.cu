@@ -190,11 +190,14 @@ cudaError_t grid_build_tets(const float4* centroid, int n_tet, const uint8_t* cl
 // ------------------------------------------------------------------------
 // cells are enumerated by `cell_at(idx)` for idx in [0, n_cells_iter), which
 // returns a cell id or -1; fn(at, valid) is called warp-uniformly for batches
-// of 32 positions in the item list (valid = false for padding lanes).
-template <class CellAt, class Fn>
+// of 32 positions in the item list (valid = false for padding lanes).  With
+// LAST one more call follows, without positions (its third argument is true):
+// the caller's code for what is left over is then in one place.
+template <bool LAST, class CellAt, class Fn>
 __device__ void for_items(int n_cells_iter, CellAt cell_at, const int32_t* cell_start, int lane,
                           Fn fn) {
-  for (int cb = 0; cb < n_cells_iter; cb += 32) {
+  for (int cb = 0; cb < n_cells_iter + (LAST ? 32 : 0); cb += 32) {
+    const bool last = LAST && cb >= n_cells_iter;
     int ci = cb + lane;
     int cell = ci < n_cells_iter ? cell_at(ci) : -1;
     int b = 0, cnt = 0;
@@ -205,7 +208,7 @@ __device__ void for_items(int n_cells_iter, CellAt cell_at, const int32_t* cell_
     int incl = warp_incl_scan<int>(cnt, lane);
     int total = __shfl_sync(0xffffffffu, incl, 31);
     int excl = incl - cnt;
-    for (int ib = 0; ib < total; ib += 32) {
+    for (int ib = 0; ib < total || (last && ib == 0); ib += 32) {
       int g = ib + lane;
       // owner lane: the last lane whose exclusive prefix is <= g
       int owner = 0;
@@ -217,7 +220,7 @@ __device__ void for_items(int n_cells_iter, CellAt cell_at, const int32_t* cell_
       int ob = __shfl_sync(0xffffffffu, b, owner);
       int oe = __shfl_sync(0xffffffffu, excl, owner);
       bool valid = g < total;
-      fn(ob + (g - oe), valid);
+      fn(ob + (g - oe), valid, last);
     }
   }
 }
@@ -432,7 +435,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == kKnnSmallWarps ? kKnnSmal
       if (x < 0 || y < 0 || z < 0 || x >= g.nx || y >= g.ny || z >= g.nz) return -1;
       return x + g.nx * (y + g.ny * z);
     };
-    for_items(n_shell, cell_at, a.cell_start, lane, [&](int at, bool valid) {
+    for_items<false>(n_shell, cell_at, a.cell_start, lane, [&](int at, bool valid, bool) {
       const int j = valid ? a.cell_items[at] : -1;
       bool take = false;
       unsigned long long packed = 0;
@@ -576,21 +579,19 @@ __device__ __forceinline__ float pow_dist(float4 s, float3 v) {
 }
 
 constexpr int kPairWarps = 4;
+// blocks that must fit an SM (72 registers); pair stage of the 1M-tet workload
+// with 5 / 6 / 7 / 8 / 9: 4.46 / 4.29 / 4.13 / 4.11 / 4.23 ms, of 5k tets 163 / 172 /
+// 169 / 170 / 178 us
+constexpr int kPairBlocks = 7;
 constexpr int kPairMaxK = 128;  // longest neighbour list (rpd_config.knn_k <= 128)
 // a tet goes through three stages, each on full warps: the centroid test
 // (one tet per lane); the tets that pass wait in a per-warp queue and try
 // the rule's first kRuleFirst neighbours 32 at a time; the tets that survive
-// those wait in a second queue and are finished 32 at a time against the
-// rest of the list (queues of kRuleQueue entries).  kRuleFirst: 4 to 16 were
-// measured on the 1M-tet workload, 8 the fastest; the macro only serves such
-// sweeps
-#ifndef RPD_RULE_FIRST
-#define RPD_RULE_FIRST 8
-#endif
-constexpr int kRuleFirst = RPD_RULE_FIRST;
-// (even: the drain steps two neighbours at a time from kRuleFirst, and its
-// acceptance checkpoints sit at multiples of 8)
-static_assert(kRuleFirst % 2 == 0, "kRuleFirst even");
+// those wait in a second queue and are finished 32 at a time against the rest
+// of the list (queues of kRuleQueue entries).  kRuleFirst: 4 to 16 were
+// measured, 8 the fastest; it and the acceptance checkpoints go by eights
+constexpr int kRuleFirst = 8;
+static_assert(kRuleFirst % 8 == 0, "groups of eight");
 constexpr int kRuleQueue = 64;
 
 // cell range of the site's box in the tet grid (empty range for no box)
@@ -616,12 +617,11 @@ __device__ __forceinline__ CellRange site_cells(const PairParams& p, int i) {
   return r;
 }
 
-// grid cells of a task: a warp works through a task alone, and one whose tets
-// all pass takes about 5 us a cell, so few sites need short tasks for the
-// other warps to help; every task stages its site's planes and list, so many
-// sites want long ones.  Pair stage (ms) with 16 / 32 / 64 / 128 / 256 / 512
-// cells: 92 sites 0.17 / 0.18 / 0.20 / 0.23 / 0.24 / 0.24, 10k sites 1.43 / 1.18 /
-// 1.20 / 1.28 / 1.62 / 1.93, 50k sites - / 5.59 / 4.89 / 4.59 / 4.59 / 5.01.
+// grid cells of a task: a warp works through a task alone, so few sites need
+// short tasks for the other warps to help; every task stages its site's planes
+// and list, so many sites want long ones.  Pair stage (ms) with 16 / 32 / 64 /
+// 128 / 256 cells: 92 sites 0.17 / 0.17 / 0.19 / 0.21 / 0.22, 10k sites 1.23 /
+// 1.05 / 1.04 / 1.12 / 1.29, 50k sites 5.81 / 4.69 / 4.29 / 4.12 / 4.18.
 int pair_task_cells(int n_site) {
   return n_site <= 512 ? 16 : (n_site <= 4096 ? 32 : (n_site <= 16384 ? 64 : 128));
 }
@@ -640,21 +640,24 @@ __global__ void pair_tasks_kernel(PairParams p, int32_t* n_tasks) {
 // or two lines.  The larger class's tets are searched with the smaller
 // class's planes pushed out further and its scaled regions (site_box_kernel):
 // 44 bisectors where its own clip took 12, so fewer tets reach the rule.  Pair
-// stage of the 1M-tet workload 5.90 -> 5.16 ms with both.
+// stage of the 1M-tet workload 5.90 -> 5.16 ms with both, 4.6 with tasks by the
+// number of sites, 4.12 with the rule's centroid test, the list staged on
+// demand and the rule's code in one place (inlined at each of its calls it
+// took 6.1: instruction fetches).
 // Persistent warps take (site, chunk of its box's cells) tasks from a work
 // counter, so a site with a large box is spread over many warps.
-__global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
+__global__ void __launch_bounds__(kPairWarps * 32, kPairBlocks) pairs_kernel(PairParams p,
                                                                 const int32_t* task_off,
                                                                 unsigned long long* work) {
   __shared__ float4 spl[kPairWarps][kBoxPlanes];
   __shared__ float spn[kPairWarps][kBoxPlanes];  // |normal| of each plane, rounded down
-  __shared__ float4 snb[kPairWarps][kPairMaxK];  // the site's neighbours (rule order)
-  // queued tets: vertices (12 floats), power distances to the site (4), and
-  // their places in the item list
-  __shared__ float sq_v[kPairWarps][16][kRuleQueue];
-  __shared__ int sq_t[kPairWarps][kRuleQueue];
-  // tets whose centroid passed, waiting for the rule's first part
+  // the site's neighbours (rule order), and their bisectors about the site
+  __shared__ float4 snb[kPairWarps][kPairMaxK];
+  __shared__ float4 sbi[kPairWarps][kPairMaxK];
+  // places in the item list: tets whose centroid passed, waiting for the
+  // rule's first part, and those that passed it, waiting for the rest
   __shared__ int sa_t[kPairWarps][kRuleQueue];
+  __shared__ int sq_t[kPairWarps][kRuleQueue];
   // every 8th neighbour r: its key and the smallest site distance |c_m - c_i|
   // (rounded down) of the neighbours from r on
   __shared__ float schk_key[kPairWarps][kPairMaxK / 8];
@@ -668,12 +671,14 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
     if (lane == 0) task = (long long)atomicAdd(work, 1ull);
     task = __shfl_sync(0xffffffffu, task, 0);
     if (task >= n_tasks) break;
-    // owning site: last i with task_off[i] <= task
+    // owning site: last i with task_off[i] <= task, 32 places at a time
     int lo = 0, hi = p.n_site - 1;
     while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if (task_off[mid] <= task) lo = mid;
-      else hi = mid - 1;
+      const int step = (hi - lo + 31) >> 5;
+      const int at = lo + (lane + 1) * step;
+      const bool below = at <= hi && __ldg(task_off + at) <= task;
+      lo += __popc(__ballot_sync(0xffffffffu, below)) * step;
+      hi = min(hi, lo + step - 1);
     }
     const int i = lo;
     const int chunk = (int)(task - task_off[i]);
@@ -716,47 +721,84 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
     // the rule is over the whole list; in ascending bisector distance (when
     // the GPU built it) the neighbour that dominates a far tet comes first
     const int32_t* L = (p.rule_nbr ? p.rule_nbr : p.nbr) + (long long)i * p.k;
-    float4* nb = snb[wid];
-    // a hole (-1) never rejects a tet: weight -inf makes its power distance +inf
+    float4 *nb = snb[wid], *bi = sbi[wid];
     const int k_staged = min(p.k, kPairMaxK);
-    for (int r = lane; r < k_staged; r += 32) {
-      const int m = __ldg(L + r);
-      nb[r] = m < 0 ? make_float4(0.f, 0.f, 0.f, -INFINITY) : __ldg(p.site4f + m);
-    }
-    __syncwarp();
-    // the acceptance checkpoints (distance-ordered lists with keys only)
     const bool acc_ok = p.rule_keys != nullptr && k_staged == p.k;
-    if (acc_ok) {
-      float carry = INFINITY;
-      for (int w = (k_staged - 1) >> 5; w >= 0; --w) {
-        const int r = lane + 32 * w;
-        float d = INFINITY;  // a hole never rejects
-        if (r < k_staged) {
-          const float4 m = nb[r];
-          if (m.w != -INFINITY) {
-            const float dx = m.x - si.x, dy = m.y - si.y, dz = m.z - si.z;
-            d = sqrtf(dx * dx + dy * dy + dz * dz) * (1.0f - 1e-6f);
-          }
+    // the list is staged for the first tet that needs it (many tasks' cells
+    // hold none)
+    bool staged = false;
+    auto stage = [&]() {
+      staged = true;
+      __syncwarp();  // the task before no longer reads its list
+      // The rule needs a vertex v with pd_m(v) > pd_i(v).  That difference is
+      // 2 (n . (v - c_i) + g), n = c_i - c_m, g = (|n|^2 + w_i - w_m) / 2:
+      // linear, so it suffices that the tet's centroid has it above the float
+      // error of the rule's own evaluation (accept_err) and of this one -- one
+      // plane test instead of four vertices.  What fails it goes through the
+      // rule itself.  g is lowered by both errors; a hole (-1) never rejects.
+      for (int r = lane; r < ((k_staged + 7) & ~7); r += 32) {
+        const int m = r < k_staged ? __ldg(L + r) : -1;
+        float4 e = make_float4(0.f, 0.f, 0.f, 1.f), sm = make_float4(0.f, 0.f, 0.f, -INFINITY);
+        if (m >= 0) {
+          sm = __ldg(p.site4f + m);
+          e.x = si.x - sm.x;
+          e.y = si.y - sm.y;
+          e.z = si.z - sm.z;
+          const float n2 = e.x * e.x + e.y * e.y + e.z * e.z;
+          const float err = 0.51f * p.accept_err + 3.0f * p.accept_margin * sqrtf(n2) +
+                            5e-7f * (n2 + fabsf(si.w) + fabsf(sm.w));
+          e.w = 0.5f * ((n2 + si.w) - sm.w) - err;
         }
-        // suffix minimum: lane l gets the minimum over lanes >= l
-        for (int o = 1; o < 32; o <<= 1) {
-          const float t = __shfl_down_sync(0xffffffffu, d, o);
-          if (lane + o < 32) d = fminf(d, t);
-        }
-        d = fminf(d, carry);
-        carry = __shfl_sync(0xffffffffu, d, 0);
-        if (r < k_staged && (r & 7) == 0) {
-          schk_d[wid][r >> 3] = d;
-          schk_key[wid][r >> 3] = __ldg(p.rule_keys + (long long)i * p.k + r);
-        }
+        bi[r] = e;
+        nb[r] = sm;
       }
       __syncwarp();
-    }
-    // neighbour r of the rule order (staged, or read for long user lists)
+      // the acceptance checkpoints (distance-ordered lists with keys only)
+      if (acc_ok) {
+        float carry = INFINITY;
+        for (int w = (k_staged - 1) >> 5; w >= 0; --w) {
+          const int r = lane + 32 * w;
+          float d = INFINITY;  // a hole never rejects
+          if (r < k_staged) {
+            const float4 e = bi[r];
+            if (nb[r].w != -INFINITY)
+              d = sqrtf(e.x * e.x + e.y * e.y + e.z * e.z) * (1.0f - 1e-6f);
+          }
+          // suffix minimum: lane l gets the minimum over lanes >= l
+          for (int o = 1; o < 32; o <<= 1) {
+            const float t = __shfl_down_sync(0xffffffffu, d, o);
+            if (lane + o < 32) d = fminf(d, t);
+          }
+          d = fminf(d, carry);
+          carry = __shfl_sync(0xffffffffu, d, 0);
+          if (r < k_staged && (r & 7) == 0) {
+            schk_d[wid][r >> 3] = d;
+            schk_key[wid][r >> 3] = __ldg(p.rule_keys + (long long)i * p.k + r);
+          }
+        }
+        __syncwarp();
+      }
+    };
+    auto centroid_passes = [&](int r, float3 y) {
+      const float4 e = bi[r];
+      return __fmaf_rn(e.x, y.x, __fmaf_rn(e.y, y.y, __fmaf_rn(e.z, y.z, e.w))) > 0.f;
+    };
+    // the rule for neighbour r: a vertex nearer to the site (in power distance)
+    auto rule = [&](const float4& sm, const float3* v, const float* pdi) {
+      bool hit = false;
+      for (int a = 0; a < 4; ++a) hit |= pow_dist(sm, v[a]) > pdi[a];
+      return hit;
+    };
     auto rule_site = [&](int r) -> float4 {
       if (r < k_staged) return nb[r];
       const int m = __ldg(L + r);
       return m < 0 ? make_float4(0.f, 0.f, 0.f, -INFINITY) : __ldg(p.site4f + m);
+    };
+    // centroid about the site
+    auto middle = [&](const float3* v) {
+      return make_float3(0.25f * (v[0].x + v[1].x + v[2].x + v[3].x) - si.x,
+                         0.25f * (v[0].y + v[1].y + v[2].y + v[3].y) - si.y,
+                         0.25f * (v[0].z + v[1].z + v[2].z + v[3].z) - si.z);
     };
     n_cells_seen += n_iter;
     // half extent of a grid cell, grown for the rounding of the binning
@@ -808,7 +850,16 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
         }
       }
     };
-    float(*qv)[kRuleQueue] = sq_v[wid];
+    // a queued tet's vertices and their power distances to the site
+    auto vertices = [&](int at, float3* v, float* pdi) {
+      const float4 q0 = __ldg(p.tcell_xyz + 3ll * at), q1 = __ldg(p.tcell_xyz + 3ll * at + 1),
+                   q2 = __ldg(p.tcell_xyz + 3ll * at + 2);
+      v[0] = make_float3(q0.x, q0.y, q0.z);
+      v[1] = make_float3(q0.w, q1.x, q1.y);
+      v[2] = make_float3(q1.z, q1.w, q2.x);
+      v[3] = make_float3(q2.y, q2.z, q2.w);
+      for (int a = 0; a < 4; ++a) pdi[a] = pow_dist(si, v[a]);
+    };
     int* qt = sq_t[wid];
     int qn = 0;  // queued tets (warp-uniform)
     // the first n queued tets, one per lane, against the rest of the list;
@@ -819,11 +870,8 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
       if (lane < n) {
         float3 v[4];
         float pdi[4];
-        for (int a = 0; a < 4; ++a) {
-          v[a] = make_float3(qv[3 * a][lane], qv[3 * a + 1][lane], qv[3 * a + 2][lane]);
-          pdi[a] = qv[12 + a][lane];
-        }
         t = qt[lane];
+        vertices(t, v, pdi);
         pass = true;
         // distance from the site to the tet's nearest vertex, rounded up
         float m2 = INFINITY;
@@ -832,35 +880,43 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
           m2 = fminf(m2, dx * dx + dy * dy + dz * dz);
         }
         const float d_up = sqrtf(m2) * (1.0f + 1e-6f);
-        for (int r = kRuleFirst; r < p.k && pass; r += 2) {
-          // pd_m(v) - pd_i(v) = 2 |c_m - c_i| (key_m - (v - c_i).u_m) for the
-          // unit direction u_m to m: a vertex within key_m of the site,
-          // by more than the float error of the two power distances, has
-          // pd_m(v) > pd_i(v) as evaluated; keys ascend along the list
-          if (acc_ok && (r & 7) == 0) {
-            const float g = schk_key[wid][r >> 3] * (1.0f - 64.0f * 5.9604645e-08f) -
-                            p.accept_margin - d_up;
-            if (g > 0.f && 2.0f * schk_d[wid][r >> 3] * g > p.accept_err) break;
+        const float3 y = middle(v);
+        bool accepted = false;
+#pragma unroll 1
+        for (int base = kRuleFirst; base < k_staged && pass && !accepted; base += 32) {
+          uint32_t fails = 0;
+#pragma unroll 1
+          for (int o = 0; o < 32 && base + o < k_staged; o += 8) {
+            const int r = base + o;
+            // pd_m(v) - pd_i(v) = 2 |c_m - c_i| (key_m - (v - c_i).u_m) for
+            // the unit direction u_m to m: a vertex within key_m of the site,
+            // by more than the float error of the two power distances, has
+            // pd_m(v) > pd_i(v) as evaluated; keys ascend along the list
+            if (acc_ok) {
+              const float g = schk_key[wid][r >> 3] * (1.0f - 64.0f * 5.9604645e-08f) -
+                              p.accept_margin - d_up;
+              if (g > 0.f && 2.0f * schk_d[wid][r >> 3] * g > p.accept_err) {
+                accepted = true;
+                break;
+              }
+            }
+#pragma unroll
+            for (int x = 0; x < 8; ++x)
+              if (!centroid_passes(r + x, y)) fails |= 1u << (o + x);
           }
-          // two neighbours per step (independent chains; the rule is an AND,
-          // so testing one past a failure changes nothing)
-          const float4 sm0 = rule_site(r);
-          const float4 sm1 = r + 1 < p.k ? rule_site(r + 1) : sm0;
-          bool hit0 = false, hit1 = false;
-          for (int a = 0; a < 4; ++a) {
-            hit0 |= pow_dist(sm0, v[a]) > pdi[a];
-            hit1 |= pow_dist(sm1, v[a]) > pdi[a];
+          while (fails && pass) {
+            const int r = base + __ffs(fails) - 1;
+            fails &= fails - 1u;
+            pass = rule(rule_site(r), v, pdi);
           }
-          pass = hit0 & hit1;
         }
+        // (long user lists beyond the staged part)
+        for (int r = k_staged; r < p.k && pass; ++r) pass = rule(rule_site(r), v, pdi);
       }
       emit(pass, t);
       __syncwarp();
       const int rest = qn - n;  // < 32: sources n.., targets 0.. do not overlap
-      if (lane < rest) {
-        for (int w = 0; w < 16; ++w) qv[w][lane] = qv[w][n + lane];
-        qt[lane] = qt[n + lane];
-      }
+      if (lane < rest) qt[lane] = qt[n + lane];
       __syncwarp();
       qn = rest;
     };
@@ -870,33 +926,27 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
     int* qa_t = sa_t[wid];
     int qa = 0;  // tets in the centroid queue (warp-uniform)
     auto first_part = [&](int n) {
+      if (!staged) stage();
       bool pass = false, survive = false;
       float3 v[4] = {};
       float pdi[4] = {};
       int t = -1;
       if (lane < n) {
         t = qa_t[lane];
-        const float4 q0 = __ldg(p.tcell_xyz + 3ll * t), q1 = __ldg(p.tcell_xyz + 3ll * t + 1),
-                     q2 = __ldg(p.tcell_xyz + 3ll * t + 2);
-        v[0] = make_float3(q0.x, q0.y, q0.z);
-        v[1] = make_float3(q0.w, q1.x, q1.y);
-        v[2] = make_float3(q1.z, q1.w, q2.x);
-        v[3] = make_float3(q2.y, q2.z, q2.w);
-        for (int a = 0; a < 4; ++a) pdi[a] = pow_dist(si, v[a]);
+        vertices(t, v, pdi);
         // voronoi.cu:154-193 (holes, -1, never reject: voronoi.cu:171):
         // a candidate iff every neighbour m has a tet vertex where
         // pd_m > pd_i; the order of the neighbours does not matter
         pass = true;
-        const int r_end = min(p.k, kRuleFirst);
-        for (int r = 0; r < r_end && pass; r += 2) {
-          const float4 sm0 = rule_site(r);
-          const float4 sm1 = r + 1 < r_end ? rule_site(r + 1) : sm0;
-          bool hit0 = false, hit1 = false;
-          for (int a = 0; a < 4; ++a) {
-            hit0 |= pow_dist(sm0, v[a]) > pdi[a];
-            hit1 |= pow_dist(sm1, v[a]) > pdi[a];
-          }
-          pass = hit0 & hit1;
+        const float3 y = middle(v);
+        uint32_t fails = 0;
+#pragma unroll
+        for (int x = 0; x < kRuleFirst; ++x)
+          if (!centroid_passes(x, y)) fails |= 1u << x;
+        while (fails && pass) {
+          const int r = __ffs(fails) - 1;
+          fails &= fails - 1u;
+          pass = rule(rule_site(r), v, pdi);
         }
         if (pass && p.k > kRuleFirst) {
           survive = true;
@@ -909,21 +959,14 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
       const uint32_t sv = __ballot_sync(0xffffffffu, survive);
       if (survive) {
         const int pos = qn + __popc(sv & ((1u << lane) - 1u));
-        for (int a = 0; a < 4; ++a) {
-          qv[3 * a][pos] = v[a].x;
-          qv[3 * a + 1][pos] = v[a].y;
-          qv[3 * a + 2][pos] = v[a].z;
-          qv[12 + a][pos] = pdi[a];
-        }
         qt[pos] = t;
       }
       qn += __popc(sv);
       emit(pass, t);
       __syncwarp();
       qa = rest;
-      if (qn >= 32) drain(32);
     };
-    for_items(n_iter, cell_at, p.tcell_start, lane, [&](int at, bool valid) {
+    for_items<true>(n_iter, cell_at, p.tcell_start, lane, [&](int at, bool valid, bool last) {
       bool in = false;
       if (valid) {
         ++n_items;
@@ -946,16 +989,17 @@ __global__ void __launch_bounds__(kPairWarps * 32) pairs_kernel(PairParams p,
         if (in) ++n_in;
       }
       // (the whole warp from here) the tets that passed join the centroid
-      // queue: qa <= 31 before, so there is room for 32 more; the rule's
-      // first part then runs on full warps
+      // queue: qa <= 31 before, so there is room for 32 more; the rule then
+      // runs on full warps, and in the last call on what is left
       const uint32_t ia = __ballot_sync(0xffffffffu, in);
       if (in) qa_t[qa + __popc(ia & ((1u << lane) - 1u))] = at;
       qa += __popc(ia);
       __syncwarp();
-      if (qa >= 32) first_part(32);
+      do {
+        if (qa >= 32 || (last && qa > 0)) first_part(min(qa, 32));
+        if (qn >= 32 || (last && qa == 0 && qn > 0)) drain(min(qn, 32));
+      } while (last && qa + qn > 0);
     });
-    if (qa > 0) first_part(qa);
-    if (qn > 0) drain(qn);
   }
   if (p.diag) {
     n_keep = __reduce_add_sync(0xffffffffu, n_keep);
