@@ -1559,13 +1559,13 @@ rpd_status rpd_compute_power_cells(rpd_ctx* c, int max_sf_fid, float* ms) {
   // neighbour pair, then by site; cells by site
   int site_bits = 1;
   while ((1ll << site_bits) < (long long)std::max(n_site, 1)) ++site_bits;
-  auto sort = [&](int k, int bits) {
+  auto sort = [&](int k, int bits, int low_bits = 32) {
     return radix_sort_pairs(keys[k], vals[k], seg[k], bits, c->pc_keys_tmp.ptr, c->pc_vals_tmp.ptr,
-                            c->pc_hist.ptr, c->pc_scan_i.ptr, st);
+                            c->pc_hist.ptr, c->pc_scan_i.ptr, st, low_bits);
   };
   CK(sort(0, 32 + site_bits), "sort");
-  CK(sort(1, 32 + site_bits), "sort");
-  CK(sort(2, 32 + site_bits), "sort");
+  CK(sort(1, 32 + site_bits, site_bits), "sort");  // (lower fields: site ids)
+  CK(sort(2, 32 + site_bits, site_bits), "sort");
   CK(pc_edges_finish(p, n_ed, 0, st), "edge keys");
   CK(sort(2, site_bits), "sort");
   CK(pc_edges_finish(p, n_ed, 1, st), "edge gather");

@@ -393,7 +393,7 @@ cudaError_t merge_gather(const long long* src, long long n, const long long* off
 size_t radix_hist_ints(long long n);
 cudaError_t radix_sort_pairs(unsigned long long* keys, uint32_t* vals, long long n, int bits,
                              unsigned long long* keys_tmp, uint32_t* vals_tmp, int32_t* hist,
-                             int32_t* scan_tmp, cudaStream_t st);
+                             int32_t* scan_tmp, cudaStream_t st, int low_bits = 32);
 
 // power cells of the emitted cells (rpd_powercell.cu)
 struct PowerCellParams {

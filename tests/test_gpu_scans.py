@@ -42,3 +42,30 @@ def test_compaction_and_offsets(n, sites):
     assert np.array_equal(th["offset"].astype(np.int64), np.cumsum(size) - size)
     assert np.all(np.diff(poly["poly_offsets"]) >= 3)
     assert poly["poly_offsets"][0] == 0 and poly["poly_offsets"][-1] == len(poly["indices"])
+
+
+@pytest.mark.parametrize("n,sites", [(2, 3), (7, 90), (20, 700), (30, 4_000)])
+def test_power_cell_records_are_sorted(n, sites):
+    """The radix sort's tiles: one, a few, many; site ids of one and two digits."""
+    cfg = W.config_small_cube(n=n, n_site=sites, seed=6)
+    adj = rpd.mesh_adjacency(cfg["vert3d"].shape[0], cfg["tets"])
+    with rpd.RPD(knn_k=24, topology_hash=False) as r:
+        r.set_mesh(cfg["vert3d"], cfg["tets"], adj["v_adjs"], adj["e_adj6"], adj["f_adjs"],
+                   adj["f_ids"])
+        r.set_sites(cfg["sites"], cfg["flags"])
+        r.compute()
+        h, _ = r.cells()
+        r.compute_topology()
+        r.compute_power_cells()
+        d = r.power_cells()
+    # cells by site, in cell order within one
+    want = np.argsort(h["site_id"], kind="stable")
+    assert np.array_equal(d["site_cells"].astype(np.int64), want)
+    # facets by (site, neighbour), then cell; each names its cell's site
+    key, cell = d["facet_keys"], d["facet_cells"].astype(np.int64)
+    assert np.array_equal(np.lexsort((cell, key)), np.arange(len(key)))
+    assert np.array_equal(key >> np.uint64(32), h["site_id"][cell].astype(np.uint64))
+    # edges (site, neighbour pair, cell, ...) by site, pair and cell
+    e = d["edges"].astype(np.int64)
+    assert np.array_equal(np.lexsort((e[:, 3], e[:, 2], e[:, 1], e[:, 0])), np.arange(len(e)))
+    assert np.array_equal(h["site_id"][e[:, 3]], e[:, 0])
