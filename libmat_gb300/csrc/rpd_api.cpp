@@ -651,25 +651,30 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
     p.ext_off = nullptr;
     p.ext_len = nullptr;
     p.ext_bound = nullptr;
+    p.ext_complete = false;
     CK(cudaEventRecord(c->ev[kEvClipK0], st), "event");
-    if (n_pairs > 0) {
-      ClipParams pw = p;
-      if (clip_threads_takes(p, c->cfg.predicate_mode)) {
-        // scratch[33], [34]: the pairs left to the general kernel, and its
-        // queue's counter
-        CK(c->ext_idx.ensure((size_t)n_pairs), "alloc ext");
-        p.back_idx = c->ext_idx.ptr;
-        CK(launch_clip_threads(p, c->cfg.predicate_mode, certify, c->num_sms, st), "clip");
-        pw.pair_index = c->ext_idx.ptr;
-        pw.n_work_dev = c->scratch.ptr + 33;
-        pw.work = c->scratch.ptr + 34;
+    // a lane per cell where the pairs are many, a warp per cell for the rest
+    // and for what outgrows the lanes (scratch[33]: those, listed in
+    // reclip_idx; [34]: their queue's counter)
+    auto clip = [&](ClipParams q, int reg_variant, int q_blocks, int q_warps) -> cudaError_t {
+      if (clip_threads_takes(q, c->cfg.predicate_mode)) {
+        cudaError_t e = cudaMemsetAsync(c->scratch.ptr + 33, 0, 2 * sizeof(unsigned long long), st);
+        if (e != cudaSuccess) return e;
+        q.back_idx = c->reclip_idx.ptr;
+        e = launch_clip_threads(q, c->cfg.predicate_mode, certify, c->num_sms, st);
+        if (e != cudaSuccess) return e;
+        q.pair_index = c->reclip_idx.ptr;
+        q.n_work_dev = c->scratch.ptr + 33;
+        q.work = c->scratch.ptr + 34;
       }
-      CK(launch_clip_cells(pw, c->cfg.predicate_mode, certify, variant, blocks, warps, st), "clip");
-    }
+      return launch_clip_cells(q, c->cfg.predicate_mode, certify, reg_variant, q_blocks, q_warps,
+                               st);
+    };
+    CK(c->reclip_idx.ensure((size_t)std::max<long long>(n_pairs, 1)), "alloc");
+    if (n_pairs > 0) CK(clip(p, variant, blocks, warps), "clip");
     CK(cudaEventRecord(c->ev[kEvClipK1], st), "event");
     if ((p.site_klen || p.pair_klen) && n_pairs > 0) {
       // cells whose shortened list was not enough: clip them again whole
-      CK(c->reclip_idx.ensure((size_t)n_pairs), "alloc");
       CK(select_pairs(c->pair_headers.ptr, n_pairs, kSecurityRadiusNotReached, c->scan_tmp.ptr,
                       c->reclip_idx.ptr, c->sel_count.ptr, st), "select");
       int32_t n_re = 0;
@@ -694,7 +699,6 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
     CK(cudaEventRecord(c->ev[kEvExt0], st), "event");
     // (scratch[32]: cells still flagged after a recheck, compacted into
     // ext_idx; the selection's count is read on the device)
-    CK(c->reclip_idx.ensure((size_t)std::max<long long>(n_pairs, 1)), "alloc");
     CK(c->ext_idx.ensure((size_t)std::max<long long>(n_pairs, 1)), "alloc");
     auto recheck = [&](bool rows) -> rpd_status {
       CK(select_uncertified(c->pair_headers.ptr, n_pairs, c->scan_tmp.ptr, c->reclip_idx.ptr,
@@ -806,8 +810,8 @@ static rpd_status finish_compute(rpd_ctx* c, bool knn, bool learned, rpd_stats* 
       pe.ext_off = c->ext_off.ptr;
       pe.ext_len = c->ext_len.ptr;
       pe.ext_bound = c->ext_bound.ptr;
-      CK(launch_clip_cells(pe, c->cfg.predicate_mode, certify, variant, blocks, warps, st),
-         "reclip extended");
+      pe.ext_complete = last;
+      CK(clip(pe, variant, blocks, warps), "reclip extended");
       ++n_ext_rounds;
       n_ext_sites += n_f;
       n_cert_reclipped += (long long)n_flag;

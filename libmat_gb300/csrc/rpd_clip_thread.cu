@@ -137,7 +137,9 @@ enum Outcome { kRun = 0, kBack = 1 };  // kBack: to clip_cells_kernel
 
 }  // namespace
 
-template <int PRED, bool CERT>
+// EXT: the re-clips of the exact-lists rounds: pairs p.pair_index[..], each with
+// its site's extended row
+template <int PRED, bool CERT, bool EXT>
 __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(ClipParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr uint32_t kAll = 0xffffffffu;
@@ -172,22 +174,24 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
   bool active = false, done = false;
   Outcome out = kRun;
   bool more = true;      // the queue has pairs left
-  const bool vec = (p.k & 3) == 0;
+  const int32_t* list = nullptr;  // the site's row
+  const float* keys = nullptr;
+  int len = p.k;
+  int row = -1;  // (EXT) its extended row
 
   auto fetch_group = [&]() {
-    const long long row = (long long)sid * p.k;
-    if (pos >= p.k) {
+    const int m = len - pos;
+    if (m <= 0) {
       jn = make_int4(-1, -1, -1, -1);
-    } else if (vec) {
-      jn = __ldg(reinterpret_cast<const int4*>(p.nbr + row + pos));
-      if (CERT) kn = __ldg(reinterpret_cast<const float4*>(p.keys + row + pos));
+    } else if (m >= 4 && (reinterpret_cast<size_t>(list + pos) & 15) == 0) {
+      jn = __ldg(reinterpret_cast<const int4*>(list + pos));
+      if (CERT) kn = __ldg(reinterpret_cast<const float4*>(keys + pos));
     } else {
-      const int32_t* l = p.nbr + row + pos;
-      const int m = p.k - pos;
+      const int32_t* l = list + pos;
       jn = make_int4(__ldg(l), m > 1 ? __ldg(l + 1) : -1, m > 2 ? __ldg(l + 2) : -1,
                      m > 3 ? __ldg(l + 3) : -1);
       if (CERT) {
-        const float* f = p.keys + row + pos;
+        const float* f = keys + pos;
         kn = make_float4(__ldg(f), m > 1 ? __ldg(f + 1) : 0.f, m > 2 ? __ldg(f + 2) : 0.f,
                          m > 3 ? __ldg(f + 3) : 0.f);
       }
@@ -242,7 +246,8 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
         if (done && out == kRun && status == kSuccess && fin == 2) {
           // the whole list without the certificate: the sites missing from
           // it have keys >= its bound (finish_list, rpd_clip.cu)
-          const float bound = p.nbr_bound ? __ldg(p.nbr_bound + sid) : INFINITY;
+          const float bound = EXT ? __ldg(p.ext_bound + row)
+                                  : (p.nbr_bound ? __ldg(p.nbr_bound + sid) : INFINITY);
           if (bound < INFINITY) {
             // finish_list's bound F exactly, unless R tells that it holds:
             // a vertex's terms of F about the seed S exceed those of eps
@@ -373,9 +378,19 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
       }
       const long long mine = base + __popc(idle & ((1u << lane) - 1u));
       if (!active && lane < p.cell_lanes && mine < p.n_work) {
-        q = (int)mine;
+        q = EXT ? __ldg(p.pair_index + mine) : (int)mine;
         t = __ldg(p.pair_tet + q);
         sid = __ldg(p.pair_site + q);
+        if (EXT) {
+          row = __ldg(p.site_row + sid);
+          const long long off = __ldg(p.ext_off + row);
+          list = p.ext_nbr + off;
+          keys = p.ext_keys + off;
+          len = __ldg(p.ext_len + row);
+        } else {
+          list = p.nbr + (long long)sid * p.k;
+          keys = p.keys + (long long)sid * p.k;
+        }
         pos = 0;
         fetch_group();
         seed = __ldg(p.site4f + sid);
@@ -739,16 +754,20 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
 // them: 17.6 pairs a tet 1260 / 1342 (id order), 475 / 843 (certified).
 constexpr long long kThreadsPairs = 20000;
 
+// The exact-lists rounds' re-clips likewise (46.6k cells with rows of up to 512
+// entries: the rounds' time 1.27 -> 1.10 ms; 10.7k cells 0.36 / 0.43 ms), but for
+// the last round, whose complete rows have no keys.
 bool clip_threads_takes(const ClipParams& p, int pred_mode) {
-  return (pred_mode == RPD_PRED_FP32_FILTER || pred_mode == RPD_PRED_EXACT) && !p.site_row &&
-         !p.site_klen && !p.pair_klen && !p.pair_index && !p.consumed && !p.lazy_cert &&
-         p.n_work >= kThreadsPairs;
+  const bool first = !p.site_row && !p.pair_index;
+  const bool again = p.site_row && p.pair_index && !p.ext_complete;
+  return (pred_mode == RPD_PRED_FP32_FILTER || pred_mode == RPD_PRED_EXACT) && (first || again) &&
+         !p.site_klen && !p.pair_klen && !p.consumed && !p.lazy_cert && p.n_work >= kThreadsPairs;
 }
 
-template <int PRED, bool CERT>
+template <int PRED, bool CERT, bool EXT>
 static cudaError_t launch_one(ClipParams p, int num_sms, cudaStream_t st) {
   const size_t smem = sizeof(WarpStore) * kTWarps;
-  cudaError_t e = cudaFuncSetAttribute(clip_threads_kernel<PRED, CERT>,
+  cudaError_t e = cudaFuncSetAttribute(clip_threads_kernel<PRED, CERT, EXT>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   // fewer pairs than lanes on the chip: fewer cells a warp, so that all of
@@ -768,18 +787,24 @@ static cudaError_t launch_one(ClipParams p, int num_sms, cudaStream_t st) {
   const long long blocks =
       std::min<long long>((long long)num_sms * kTBlocks, (p.n_work + per_block - 1) / per_block);
   if (blocks < 1) return cudaSuccess;
-  clip_threads_kernel<PRED, CERT><<<(unsigned)blocks, kTWarps * 32, smem, st>>>(p);
+  clip_threads_kernel<PRED, CERT, EXT><<<(unsigned)blocks, kTWarps * 32, smem, st>>>(p);
   note_launches(1);
   return cudaGetLastError();
+}
+
+template <int PRED, bool CERT>
+static cudaError_t launch_list(const ClipParams& p, int num_sms, cudaStream_t st) {
+  return p.site_row ? launch_one<PRED, CERT, true>(p, num_sms, st)
+                    : launch_one<PRED, CERT, false>(p, num_sms, st);
 }
 
 cudaError_t launch_clip_threads(const ClipParams& p, int pred_mode, int certify, int num_sms,
                                 cudaStream_t st) {
   if (pred_mode == RPD_PRED_EXACT)
-    return certify ? launch_one<RPD_PRED_EXACT, true>(p, num_sms, st)
-                   : launch_one<RPD_PRED_EXACT, false>(p, num_sms, st);
-  return certify ? launch_one<RPD_PRED_FP32_FILTER, true>(p, num_sms, st)
-                 : launch_one<RPD_PRED_FP32_FILTER, false>(p, num_sms, st);
+    return certify ? launch_list<RPD_PRED_EXACT, true>(p, num_sms, st)
+                   : launch_list<RPD_PRED_EXACT, false>(p, num_sms, st);
+  return certify ? launch_list<RPD_PRED_FP32_FILTER, true>(p, num_sms, st)
+                 : launch_list<RPD_PRED_FP32_FILTER, false>(p, num_sms, st);
 }
 
 }  // namespace rpd

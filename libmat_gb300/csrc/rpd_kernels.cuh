@@ -81,6 +81,7 @@ struct ClipParams {
   const long long* ext_off;
   const int32_t* ext_len;
   const float* ext_bound;
+  bool ext_complete;             // the rows hold every site, in id order, without keys
 };
 
 // cells flagged RPD_CELL_UNCERTIFIED by the clip kernel, bounded again:

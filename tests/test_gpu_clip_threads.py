@@ -121,3 +121,17 @@ def test_exact_signs_equal_the_oracle(n, m):
                 **{k: adj[k] for k in ("v_adjs", "e_adj6", "f_adjs", "f_ids")})
     oh, op, _ = O.clip_cells(mesh, cfg["sites"], nbr, offs, ps, pred_mode=2)
     assert same_records(ph, p, oh, op)
+
+
+@pytest.mark.parametrize("certify", [False, True])
+def test_extended_rows_equal_fp64_path(certify):
+    """Short base lists: the exact-lists rounds clip enough cells again for the
+    lanes, with rows of up to 512 entries at odd places."""
+    cfg = W.config_small_cube(n=20, n_site=2_000, seed=5)
+    adj = rpd.mesh_adjacency(cfg["vert3d"].shape[0], cfg["tets"])
+    a, ha, (_, pa), ta = run(cfg, adj, rpd.PRED_FP64, knn_k=14, certify=certify)
+    b, hb, (_, pb), tb = run(cfg, adj, rpd.PRED_FP32_FILTER, knn_k=14, certify=certify)
+    assert b.n_cert_reclipped >= MIN_PAIRS and a.n_uncertified == b.n_uncertified == 0
+    assert np.array_equal(ha["status"], hb["status"]) and np.array_equal(ta, tb)
+    if not certify:
+        assert same_records(ha, pa, hb, pb)
