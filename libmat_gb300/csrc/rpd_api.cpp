@@ -972,7 +972,9 @@ rpd_status rpd_compute(rpd_ctx* c, rpd_stats* stats) {
     // the nearest bisectors bound each cell; with a GPU-built list the
     // distance-ordered copy gives them first, a user list is used whole
     const int32_t* box_list = knn ? c->nbr_dist.ptr : c->nbr.ptr;
-    const int box0 = c->cfg.box_planes > 0 ? c->cfg.box_planes : kDefaultBoxPlanes;
+    const int box0 = c->cfg.box_planes > 0
+                         ? c->cfg.box_planes
+                         : default_box_planes(n_site, c->w_max, c->mesh_lo, c->mesh_hi);
     CK(c->site_box.ensure((size_t)n_site * 2), "alloc");
     CK(c->site_box1.ensure((size_t)n_site * 2), "alloc");
     CK(c->t_cell_cent.ensure((size_t)n_tet), "alloc");

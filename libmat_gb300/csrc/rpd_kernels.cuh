@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 
@@ -149,10 +151,26 @@ struct BoxParams {
 
 constexpr int kBoxPlanes = 48;
 // nearest bisectors that bound each site's candidate region for the tets of
-// common size (rpd_config.box_planes = 0); measured on the 1M-tet ellipsoid:
-// 32 -> 9.07 ms, 40 -> 8.72, 44 -> 8.60, 48 -> 8.65, 56 -> 9.29 ms for the
-// pair search
-constexpr int kDefaultBoxPlanes = 44;
+// common size (rpd_config.box_planes = 0), by the number of sites: each costs
+// every site's clip the same, and the tighter region pays in the pair search,
+// which grows with the sites (and their crowding).  Pair stage (ms) with 12 /
+// 16 / 24 / 32 / 44: 92 sites 0.134 / 0.142 / 0.150 / 0.160 / 0.170, 2k 0.219 /
+// 0.215 / 0.232 / 0.242 / 0.261, 4k 0.80 / 0.65 / 0.55 / 0.53 / 0.54, 10k 2.00 / 1.40 /
+// 1.07 / 1.01 / 1.04, 50k 18.4 / 10.1 / 5.30 / 4.45 / 4.16.  Where the largest weight
+// is small against the spacing of the sites, so that a cell's nearest sites
+// bound it, few do (3.4k equal lattice sites 0.25 / 0.27 / 0.30 / 0.31 / 0.32; 24
+// meshes of uniform sites, front end 2.9 / 3.0 / 3.4 / 3.7 / 4.2): below 0.4 of the
+// squared spacing (0.3 and 0.6 measure the same, 1.0 takes the 10k sites in).
+inline int default_box_planes(int n_site, double w_max, const double* lo, const double* hi) {
+  const int planes = n_site <= 512     ? 12
+                     : n_site <= 2048  ? 16
+                     : n_site <= 8192  ? 24
+                     : n_site <= 20000 ? 32
+                                       : 44;
+  const double volume = (hi[0] - lo[0]) * (hi[1] - lo[1]) * (hi[2] - lo[2]);
+  const double spacing = std::cbrt(std::max(volume, 0.0) / std::max(n_site, 1));
+  return w_max < 0.4 * spacing * spacing ? std::min(planes, 16) : planes;
+}
 
 size_t clip_smem_per_warp();
 int clip_blocks_per_sm(int pred_mode, int warps);
