@@ -100,8 +100,9 @@ typedef struct rpd_config {
                             clipped again with the whole list */
   int box_planes;        /* RPD_NEIGH_KNN: nearest bisectors bounding each
                             site's candidate region for the tets of common
-                            size (0 = default 44; the few largest tets use
-                            at most 12) */
+                            size (0 = default: 12 to 44 by the number of
+                            sites and their weights; the few largest tets
+                            use at most 12 of their own) */
   int topology_hash;     /* 1 (default): canonical topology hash of every
                             cell (rpd_copy_topology_hashes_to_host) */
   int exact_lists;       /* 1 (default; RPD_NEIGH_KNN): a site whose cell

@@ -11,7 +11,7 @@
 // lines).
 //
 // Measured (1M tets, 50k sites, 4.05M pairs, certified lists of 128): 18.2 ms
-// a warp per cell, 5.5 ms here with the 1.6 % of the pairs that go back.  What
+// a warp per cell, 5.4 ms here with the 1.1 % of the pairs that go back.  What
 // bounds it is issue and latency: the phases run with 12 to 20 of 32 lanes, and
 // twelve warps an SM hide only part of the shared-memory and list loads.
 //
@@ -749,7 +749,7 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
 // kThreadsPairs pairs on.  Below, one lane's serial clips take longer than a
 // warp's (clip stage, us, thread / warp per cell): 14k pairs 112 / 78 (id
 // order) and 68 / 80 (certified), 25k 170 / 193 and 143 / 162, 195k
-// 475 / 1350, 4.05M (certified) 5470 / 18180.  Cells of many planes (many
+// 475 / 1350, 4.05M (certified) 5400 / 18180.  Cells of many planes (many
 // sites in few tets) still gain, although the warps take back up to half of
 // them: 17.6 pairs a tet 1260 / 1342 (id order), 475 / 843 (certified).
 constexpr long long kThreadsPairs = 20000;
@@ -774,11 +774,12 @@ static cudaError_t launch_one(ClipParams p, int num_sms, cudaStream_t st) {
   // its warps work and their lanes diverge less
   const long long warps = (long long)num_sms * kTBlocks * kTWarps;
   p.cell_lanes = (int)std::min<long long>(32, std::max<long long>(4, (p.n_work + warps - 1) / warps));
-  // of 32 lanes, swept on the 1M-tet workload (clip stage, ms): new pairs at
-  // 4 / 8 / 12 / 16 / 24 idle ones 9.1 / 8.4 / 8.0 / 7.7 / 7.7, clipping below
-  // 4 / 8 / 12 / 16 scanning ones 7.9 / 7.7 / 7.8 / 8.1; undecided signs end
-  // in the filter mostly (1 / 2 / 8 / 24 lanes 5.45 / 5.47 / 5.75 / 5.89), in
-  // expansions on exact ties (146k-tet lattice: 13.2 / 12.7 / 9.8 / 8.3)
+  // of 32 lanes, swept on the 1M-tet workload (clip stage, ms; the first two
+  // before the box culling): new pairs at 4 / 8 / 12 / 16 / 24 idle ones 9.1 /
+  // 8.4 / 8.0 / 7.7 / 7.7, clipping below 4 / 8 / 12 / 16 scanning ones 7.9 / 7.7 /
+  // 7.8 / 8.1; undecided signs end in the filter mostly (1 / 2 / 8 / 24 lanes
+  // 5.45 / 5.47 / 5.75 / 5.89), in exact arithmetic on exact ties (146k-tet
+  // lattice, by expansions: 13.2 / 12.7 / 9.8 / 8.3)
   auto part = [&](int of32) { return std::max(1, p.cell_lanes * of32 / 32); };
   p.refill_lanes = part(16);
   p.scan_lanes = part(8);
