@@ -191,14 +191,14 @@ def clip_algorithmic_bytes(cfg, n_pairs, k, topo_bytes):
 
 
 # DRAM traffic of one clip launch per candidate pair: ncu
-# dram__bytes_read.sum + dram__bytes_write.sum of clip_cells_kernel on the
+# dram__bytes_read.sum + dram__bytes_write.sum of clip_threads_kernel on the
 # 200k-tet ellipsoid (the same workload family, scaled by the launch's pairs:
 # its traffic grows with them), and smsp__issue_active of the same capture;
 # the capture and its command are summarised in
-# profiles/clip_cells_kernel_ellipsoid_200k.md
-CLIP_DRAM_BYTES_PER_PAIR = 320.9
-CLIP_ISSUE_ACTIVE = 0.695
-CLIP_THREADS_PER_INST = 16.27
+# profiles/clip_threads_kernel_ellipsoid_200k.md
+CLIP_DRAM_BYTES_PER_PAIR = 304.1
+CLIP_ISSUE_ACTIVE = 0.499
+CLIP_THREADS_PER_INST = 14.18
 
 
 def sample_tets(n_tet, n, seed):
@@ -632,7 +632,7 @@ def run_ours(args):
         "e2e": e2e,
         "topology": topology,
         "gpu_launches": int(st.n_launches) * args.steps,
-        "roofline": {"bound": "hbm", "kernel": "clip_cells_kernel", "achieved": achieved,
+        "roofline": {"bound": "hbm", "kernel": "clip_threads_kernel", "achieved": achieved,
                      "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                      "peak_source": peak_src,
                      "algorithmic_bytes": alg,
