@@ -85,6 +85,13 @@ __device__ __forceinline__ float det3x3_f(float4 a, float4 b, float4 c) {
 // the reference's FP64 evaluation (gamma_9 in double times the 4x4
 // permanent), so a decided sign is the sign of the reference's FP64 det.
 // ------------------------------------------------------------------------
+// A result below 2^-126 is rounded to a multiple of 2^-149, whatever its size:
+// the 2x2 minors are then off by up to 2^-149 and the determinant by
+// 2^-149 (|a1| + |b1| + |c1|) + 3 2^-150 more than in proportion to the
+// permanent.  The permanents therefore start from kMinorFloor in place of
+// zero, which in 6 u times them is at least four times that, and they stay
+// clear of the subnormals themselves (above 2^-100 the floor does not show).
+constexpr float kMinorFloor = 2.3509887e-38f;  // 2^-125
 __device__ __forceinline__ void minor3(float a1, float b1, float c1, float a2,
                                        float b2, float c2, float a3, float b3,
                                        float c3, float& det, float& perm) {
@@ -92,10 +99,11 @@ __device__ __forceinline__ void minor3(float a1, float b1, float c1, float a2,
   float u2 = __fmaf_rn(a2, c3, -(a3 * c2));
   float u3 = __fmaf_rn(a2, b3, -(a3 * b2));
   det = __fmaf_rn(a1, u1, __fmaf_rn(-b1, u2, c1 * u3));
-  float v1 = __fmaf_rn(fabsf(b2), fabsf(c3), fabsf(b3) * fabsf(c2));
-  float v2 = __fmaf_rn(fabsf(a2), fabsf(c3), fabsf(a3) * fabsf(c2));
-  float v3 = __fmaf_rn(fabsf(a2), fabsf(b3), fabsf(a3) * fabsf(b2));
-  perm = __fmaf_rn(fabsf(a1), v1, __fmaf_rn(fabsf(b1), v2, fabsf(c1) * v3));
+  float v1 = __fmaf_rn(fabsf(b2), fabsf(c3), __fmaf_rn(fabsf(b3), fabsf(c2), kMinorFloor));
+  float v2 = __fmaf_rn(fabsf(a2), fabsf(c3), __fmaf_rn(fabsf(a3), fabsf(c2), kMinorFloor));
+  float v3 = __fmaf_rn(fabsf(a2), fabsf(b3), __fmaf_rn(fabsf(a3), fabsf(b2), kMinorFloor));
+  perm = __fmaf_rn(fabsf(a1), v1,
+                   __fmaf_rn(fabsf(b1), v2, __fmaf_rn(fabsf(c1), v3, kMinorFloor)));
 }
 
 __device__ __forceinline__ void vertex_cofactors(float4 p1, float4 p2, float4 p3,

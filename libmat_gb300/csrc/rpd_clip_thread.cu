@@ -86,7 +86,9 @@ __device__ __forceinline__ float4 make_vertex(float4 p1, float4 p2, float4 p3, f
   const float ew = g * M.w, aw = -K.w;
   float x = 0.f, y = 0.f, z = 0.f;
   uint32_t code = kEpsInf;
-  if (aw > 2.0f * ew) {  // else (or K_w > 0) every test of it goes to the filter
+  // else (or K_w > 0, or too small to divide by with the error taken below)
+  // every test of it goes to the filter
+  if (aw > __fmaf_rn(2.0f * g, M.w, 1e-36f)) {
     const float nx = __fmaf_rn(aw, c.x, K.x), ny = __fmaf_rn(aw, c.y, K.y),
                 nz = __fmaf_rn(aw, c.z, K.z);
     const float e = g * (M.x + M.y + M.z + (fabsf(c.x) + fabsf(c.y) + fabsf(c.z)) * M.w) +

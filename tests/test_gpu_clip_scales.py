@@ -1,0 +1,43 @@
+"""The clippers on scenes scaled by powers of two.  The planes' minors then fall
+through the range of the single precision's subnormals, where an error is not
+in proportion to the terms any more; every sign has to stay the sign of the
+reference's FP64 determinant (which no such scale touches), with a lane and
+with a warp per cell.  Scaling changes no plane's float mantissa as long as
+nothing underflows, so the FP64 path, the oracle and the unscaled scene are all
+references."""
+import numpy as np
+import pytest
+
+from libmat_gb300 import rpd
+from libmat_gb300 import workloads as W
+from tests.helpers import SUCCESS
+from tests.test_gpu_clip_threads import MIN_PAIRS, run, same_records
+
+pytestmark = pytest.mark.gpu
+
+
+def scaled(cfg, k):
+    """The scene in a frame of 1000 x 2^-k units."""
+    s = np.ldexp(1.0, -k)
+    return dict(cfg, vert3d=cfg["vert3d"] * s, sites=cfg["sites"] * np.array([s, s, s, s * s]))
+
+
+SIZES = {"lanes": (20, 2_000), "warps": (8, 250)}  # pairs above and below MIN_PAIRS
+
+
+def scene(size):
+    n, sites = SIZES[size]
+    cfg = W.config_small_cube(n=n, n_site=sites, seed=5)
+    return cfg, rpd.mesh_adjacency(cfg["vert3d"].shape[0], cfg["tets"])
+
+
+@pytest.mark.parametrize("size", ["lanes", "warps"])
+@pytest.mark.parametrize("k", [10, 20, 24, 25, 26, 27, 29, 30])
+def test_filtered_signs_equal_fp64_path(size, k):
+    cfg, adj = scene(size)
+    cfg = scaled(cfg, k)
+    a, ha, (_, pa), _ = run(cfg, adj, rpd.PRED_FP64, knn_k=64, exact_lists=False)
+    b, hb, (_, pb), _ = run(cfg, adj, rpd.PRED_FP32_FILTER, knn_k=64, exact_lists=False)
+    assert (b.n_pairs >= MIN_PAIRS) == (size == "lanes") and b.n_pairs == a.n_pairs
+    assert (ha["status"] == SUCCESS).mean() > 0.5
+    assert same_records(ha, pa, hb, pb)
