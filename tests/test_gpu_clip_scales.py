@@ -10,6 +10,7 @@ import pytest
 
 from libmat_gb300 import rpd
 from libmat_gb300 import workloads as W
+from oracle import oracle as O
 from tests.helpers import SUCCESS
 from tests.test_gpu_clip_threads import MIN_PAIRS, run, same_records
 
@@ -41,3 +42,25 @@ def test_filtered_signs_equal_fp64_path(size, k):
     assert (b.n_pairs >= MIN_PAIRS) == (size == "lanes") and b.n_pairs == a.n_pairs
     assert (ha["status"] == SUCCESS).mean() > 0.5
     assert same_records(ha, pa, hb, pb)
+
+
+@pytest.mark.parametrize("n,m", [(14, 7), (8, 4)])  # pairs above and below MIN_PAIRS
+@pytest.mark.parametrize("k", [10, 24, 25, 26, 27, 28, 29])
+def test_exact_signs_equal_the_oracle(n, m, k):
+    """Ties of lattice sites, which FP64 leaves undecided at every scale."""
+    cfg = W.config_lattice(n=n, m=m)
+    adj = rpd.mesh_adjacency(cfg["vert3d"].shape[0], cfg["tets"])
+    cfg = scaled(cfg, k)
+    with rpd.RPD(predicate_mode=rpd.PRED_EXACT, knn_k=40, exact_lists=False) as r:
+        r.set_mesh(cfg["vert3d"], cfg["tets"], adj["v_adjs"], adj["e_adj6"], adj["f_adjs"],
+                   adj["f_ids"])
+        r.set_sites(cfg["sites"], cfg["flags"])
+        st = r.compute()
+        nbr = r.neighbor_lists(len(cfg["sites"]))
+        offs, ps = r.pairs(len(cfg["tets"]))
+        ph, p = r.pair_headers(), r.cells()[1]
+    assert (st.n_pairs >= MIN_PAIRS) == (n == 14) and st.n_fp64_uncertain > 0
+    mesh = dict(vert3d=cfg["vert3d"], tets=cfg["tets"],
+                **{q: adj[q] for q in ("v_adjs", "e_adj6", "f_adjs", "f_ids")})
+    oh, op, _ = O.clip_cells(mesh, cfg["sites"], nbr, offs, ps, pred_mode=2)
+    assert same_records(ph, p, oh, op)
