@@ -394,8 +394,18 @@ __device__ __forceinline__ float vertex_radius(float4 K, float4 M, float3 S) {
   float ey = g * (M.y + fabsf(S.y) * M.w) + 2.4e-7f * fabsf(ny);
   float ez = g * (M.z + fabsf(S.z) * M.w) + 2.4e-7f * fabsf(nz);
   float ax = fabsf(nx) + ex, ay = fabsf(ny) + ey, az = fabsf(nz) + ez;
-  float num = sqrtf(ax * ax + ay * ay + az * az) * (1.0f + 1e-6f);
-  return num / (aw - ew) * (1.0f + 1e-6f);
+  const float n2 = ax * ax + ay * ay + az * az;
+  float n = sqrtf(n2);
+  if (n2 < 1e-30f) {
+    // the squares underflow, to a radius of zero that certifies any cell
+    // (48k tets in 1e-3 units and less; some vertices from 3e-2 down)
+    constexpr float up = 1.2676506e30f;  // 2^100
+    ax *= up;
+    ay *= up;
+    az *= up;
+    n = sqrtf(ax * ax + ay * ay + az * az) * (1.0f / up);
+  }
+  return n * (1.0f + 1e-6f) / (aw - ew) * (1.0f + 1e-6f);
 }
 
 // The same bound in FP64, for a vertex whose FP32 bound is loose or void

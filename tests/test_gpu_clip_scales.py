@@ -64,3 +64,21 @@ def test_exact_signs_equal_the_oracle(n, m, k):
                 **{q: adj[q] for q in ("v_adjs", "e_adj6", "f_adjs", "f_ids")})
     oh, op, _ = O.clip_cells(mesh, cfg["sites"], nbr, offs, ps, pred_mode=2)
     assert same_records(ph, p, oh, op)
+
+
+@pytest.mark.parametrize("size", ["lanes", "warps"])
+@pytest.mark.parametrize("pred", ["fp64", "fp32_filter", "exact"])
+@pytest.mark.parametrize("certify", [False, True])
+def test_certified_topology_as_unscaled(size, pred, certify):
+    """The radius bounds behind the certificate and the uncertified flags: short
+    lists, so that the exact-lists rounds have cells to complete.  A topology
+    hash is made of ids, which no scale changes."""
+    cfg, adj = scene(size)
+    mode = {"fp64": rpd.PRED_FP64, "fp32_filter": rpd.PRED_FP32_FILTER, "exact": rpd.PRED_EXACT}[pred]
+    a, ha, _, ta = run(cfg, adj, rpd.PRED_FP64, knn_k=24, certify=certify)
+    assert a.n_extended_sites > 0 and a.n_uncertified == 0
+    for k in (10, 15, 17, 20, 23, 25, 27, 29):
+        b, hb, _, tb = run(scaled(cfg, k), adj, mode, knn_k=24, certify=certify)
+        assert b.n_uncertified == 0, k
+        assert np.array_equal(ha["status"], hb["status"]), k
+        assert np.array_equal(ta, tb), k
