@@ -39,6 +39,7 @@
 
 #include <algorithm>
 
+#include "rpd_clip_box.cuh"
 #include "rpd_clip_pred.cuh"
 #include "rpd_common.cuh"
 #include "rpd_kernels.cuh"
@@ -155,8 +156,8 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
   float3 c = make_float3(0.f, 0.f, 0.f);
   float cmag = 0.f;      // |c|
   float span = 0.f;      // largest |x'|
-  float3 mid = c, half = c;  // box of the vertices (about c), eps and a slack included
-  float R = 0.f;         // radius about the seed, slack included
+  CullBox box = {c, c, 0.f};  // box of the vertices (about c) and their radius about
+                              // the seed, eps and a slack included
   int np = 0, nv = 0, ne = 0, status = kSuccess, pos = 0;
   uint32_t h4 = 0;       // #adjacent of the tet's faces
   int4 jn = make_int4(-1, -1, -1, -1);  // the next group of the list
@@ -199,11 +200,10 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
       }
     }
   };
-  // span, the box, and R of the vertices.  The box and R take a slack of
-  // 2^-10 span, so that a clip's new vertices (their eps) stay inside those
-  // the cull of a group used; true if one does not: a clip shrinks the cell,
-  // but where signs are ties a vertex of three nearly dependent planes can
-  // land outside it
+  // span and box of the vertices.  The box takes a slack of 2^-10 span, so that
+  // a clip's new vertices (their eps) stay inside the one the cull of a group
+  // used; true if one does not: a clip shrinks the cell, but where signs are
+  // ties a vertex of three nearly dependent planes can land outside it
   auto bounds = [&]() {
     const float sx = c.x - seed.x, sy = c.y - seed.y, sz = c.z - seed.z;
     float d2 = 0.f, s2 = 0.f, em = 0.f;
@@ -223,14 +223,7 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
     span = sqrt_fast(d2) * (1.0f + 2e-6f);
     const float r = (sqrt_fast(s2) + em) * (1.0f + 2e-6f) +
                     3e-7f * (span + fabsf(sx) + fabsf(sy) + fabsf(sz));
-    const bool outside = lo.x < mid.x - half.x || hi.x > mid.x + half.x || lo.y < mid.y - half.y ||
-                         hi.y > mid.y + half.y || lo.z < mid.z - half.z ||
-                         hi.z > mid.z + half.z || r > R;
-    const float slack = span * (1.0f / 1024.0f);
-    R = r + slack;
-    mid = make_float3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
-    half = make_float3(0.5f * (hi.x - lo.x) + slack, 0.5f * (hi.y - lo.y) + slack,
-                       0.5f * (hi.z - lo.z) + slack);
+    const bool outside = fit_box(box, lo, hi, r, span * (1.0f / 1024.0f));
     // a sliver's vertex whose place is hardly known would send every test of
     // it to the filter, one lane at a time
     if (!(em < 0.25f * span)) out = kBack;
@@ -260,8 +253,8 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
             const float c1 = fabsf(c.x) + fabsf(c.y) + fabsf(c.z);
             float em = 0.f;
             for (int v = 0; v < nv; ++v) em = fmaxf(em, eps_of(w.vx[v][lane].w));
-            const float F = R * (1.0f + 1e-6f) +
-                            1.1f * em * (1.0f + __fdividef(s1 + 2.0f * R, c1));
+            const float F = box.R * (1.0f + 1e-6f) +
+                            1.1f * em * (1.0f + __fdividef(s1 + 2.0f * box.R, c1));
             if (!cert_holds(bound, F, p.cert_margin))
               uncert = !cert_holds(
                   bound, fresh_radius(w, lane, nv, make_float3(seed.x, seed.y, seed.z)),
@@ -423,9 +416,9 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
         nv = 0;
         ne = 6;
         want = 4;  // its vertices
-        mid = make_float3(0.f, 0.f, 0.f);
-        half = make_float3(INFINITY, INFINITY, INFINITY);
-        R = INFINITY;
+        box.mid = make_float3(0.f, 0.f, 0.f);
+        box.half = make_float3(INFINITY, INFINITY, INFINITY);
+        box.R = INFINITY;
         status = kSuccess;
         out = kRun;
         cand = 0;
@@ -571,16 +564,17 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
           for (int u = 0; u < 4; ++u) {
             if (fin == 0 && u >= skip) {
               if (js[u] < 0) fin = 2;
-              else if (CERT && cert_holds(ks[u], R, p.cert_margin)) fin = 1;
+              else if (CERT && cert_holds(ks[u], box.R, p.cert_margin)) fin = 1;
             }
             const float4 f = bisector_f(seed, B[u]);
             const float n2 = __fmaf_rn(f.x, f.x, __fmaf_rn(f.y, f.y, f.z * f.z));
             const float nn = sqrt_fast(n2) * (1.0f + 1e-6f);
             const float wp = __fmaf_rn(f.x, c.x, __fmaf_rn(f.y, c.y, __fmaf_rn(f.z, c.z, f.w)));
             const float at = __fmaf_rn(
-                f.x, mid.x, __fmaf_rn(f.y, mid.y, __fmaf_rn(f.z, mid.z, wp)));
+                f.x, box.mid.x, __fmaf_rn(f.y, box.mid.y, __fmaf_rn(f.z, box.mid.z, wp)));
             const float ext = __fmaf_rn(
-                fabsf(f.x), half.x, __fmaf_rn(fabsf(f.y), half.y, fabsf(f.z) * half.z));
+                fabsf(f.x), box.half.x,
+                __fmaf_rn(fabsf(f.y), box.half.y, fabsf(f.z) * box.half.z));
             const float tol =
                 4.8e-7f * __fmaf_rn(nn, cmag + 5.0f * span, fabsf(f.w)) + 1e-30f;
             const bool clear = n2 > 1e-25f && at - ext > tol;
