@@ -151,7 +151,12 @@ typedef struct rpd_stats {
   int64_t n_pairs;            /* candidate (tet, site) pairs clipped */
   int64_t n_cells;            /* emitted cells (status success) */
   int64_t status_counts[10];  /* per reference status value 0..8, [9] other */
-  int64_t n_predicates;       /* conflict predicates evaluated */
+  int64_t n_predicates;       /* conflict predicates evaluated, over the clips
+                                 that made the cells and those of earlier
+                                 rounds (n_reclipped, n_cert_reclipped).  The
+                                 thread-per-cell clipper passes over planes
+                                 that a box of the cell clears: those are not
+                                 counted, so its rate of escalations is higher */
   int64_t n_escalated;        /* of those, decided by the FP64 determinant */
   int64_t payload_bytes;      /* payload bytes written */
   int32_t tet_k;              /* max pairs of one tet (reference's tet_k) */

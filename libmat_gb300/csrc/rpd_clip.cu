@@ -115,7 +115,14 @@ __device__ __forceinline__ bool in_conflict(const WarpCell& c, int vi, float4 e,
     if (s != 0) return s > 0;
     ++pc.esc;
     const uchar4 v = c.ver[vi];
-    if (PRED == RPD_PRED_EXACT) return exact_conflict(c.pl[v.x], c.pl[v.y], c.pl[v.z], e, c.u.f.M[vi], pc.exact);
+    if (PRED == RPD_PRED_EXACT) {
+      const int x = exact_conflict(c.pl[v.x], c.pl[v.y], c.pl[v.z], e, c.u.f.M[vi]);
+      if (pc.exact && (x & kSignUncertain)) {
+        atomicAdd(pc.exact, 1ull);
+        if (x & kSignFlip) atomicAdd(pc.exact + 1, 1ull);
+      }
+      return x & kSignConflict;
+    }
     return det4x4_ref(c.pl[v.x], c.pl[v.y], c.pl[v.z], e) > 0.0;
   }
   return det4x4_of(load_minors(c, vi), e) > 0.0;

@@ -356,18 +356,17 @@ __host__ __device__ constexpr bool uses_filter(int pred) {
 }
 
 // RPD_PRED_EXACT: the predicates the filter cannot decide, out of line
-// (rare); M the permanents of the three planes.  counts (optional): [0] FP64
-// signs not certified by their error bound (decided exactly), [1] exact signs
-// different from the FP64 sign
-static __device__ __noinline__ bool exact_conflict(float4 p1, float4 p2, float4 p3, float4 e,
-                                                   float4 M, unsigned long long* counts) {
+// (rare); M the permanents of the three planes.  kSignConflict where they
+// conflict, kSignUncertain where the FP64 sign is not certified by its error
+// bound (decided exactly), kSignFlip where the exact sign differs from it
+enum SignBits { kSignConflict = 1, kSignUncertain = 2, kSignFlip = 4, kSignEscalated = 8 };
+static __device__ __noinline__ int exact_conflict(float4 p1, float4 p2, float4 p3, float4 e,
+                                                  float4 M) {
   const double d = det4x4_ref(p1, p2, p3, e);
-  if (fabs(d) > det4x4_bound(M, e)) return d > 0.0;
-  if (counts) atomicAdd(counts, 1ull);
+  if (fabs(d) > det4x4_bound(M, e)) return d > 0.0 ? kSignConflict : 0;
   int xs = det4x4_sum_sign(p1, p2, p3, e);
   if (xs == 2) xs = det4x4_exact_sign(p1, p2, p3, e);
-  if (counts && (xs > 0) != (d > 0.0)) atomicAdd(counts + 1, 1ull);
-  return xs > 0;
+  return kSignUncertain | (xs > 0 ? kSignConflict : 0) | ((xs > 0) != (d > 0.0) ? kSignFlip : 0);
 }
 
 // ------------------------------------------------------------------------

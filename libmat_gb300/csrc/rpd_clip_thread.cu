@@ -106,20 +106,18 @@ __device__ __forceinline__ float4 make_vertex(float4 p1, float4 p2, float4 p3, f
   return make_float4(x, y, z, __uint_as_float(bits | (code << 20)));
 }
 
-// a sign the positions cannot decide
+// a sign the positions cannot decide (SignBits)
 template <int PRED>
-__device__ __noinline__ bool slow_conflict(float4 p1, float4 p2, float4 p3, float4 e,
-                                           unsigned long long* exact, uint32_t* esc) {
+__device__ __noinline__ int slow_conflict(float4 p1, float4 p2, float4 p3, float4 e) {
   // on a plane identical to e the vertex is no conflict (its value is zero,
   // which the filters cannot decide: every such test arrives here)
-  if (plane_eq(e, p1) || plane_eq(e, p2) || plane_eq(e, p3)) return false;
+  if (plane_eq(e, p1) || plane_eq(e, p2) || plane_eq(e, p3)) return 0;
   float4 K, M;
   vertex_cofactors(p1, p2, p3, K, M);
   const int s = filter_sign(K, M, e);
-  if (s != 0) return s > 0;
-  ++*esc;
-  if (PRED == RPD_PRED_EXACT) return exact_conflict(p1, p2, p3, e, M, exact);
-  return det4x4_ref(p1, p2, p3, e) > 0.0;
+  if (s != 0) return s > 0 ? kSignConflict : 0;
+  if (PRED == RPD_PRED_EXACT) return kSignEscalated | exact_conflict(p1, p2, p3, e, M);
+  return kSignEscalated | (det4x4_ref(p1, p2, p3, e) > 0.0 ? kSignConflict : 0);
 }
 
 // the radius bound finish_list tests (rpd_clip.cu): the largest of the
@@ -149,6 +147,11 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
   const int lane = threadIdx.x & 31;
   WarpStore& w = reinterpret_cast<WarpStore*>(smem_raw)[threadIdx.x >> 5];
   uint32_t n_pred = 0, n_esc = 0;
+  // the lane's cell's predicates, escalations and exact signs: they count only
+  // if it ends here (clip_cells_kernel counts those it takes up again)
+  struct {
+    uint32_t pred, esc, uncertain, flips;
+  } cell = {0u, 0u, 0u, 0u};
 
   // the lane's cell
   int q = -1, t = 0, sid = 0;
@@ -275,6 +278,12 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
         if (done && out == kBack) {
           p.back_idx[atomicAdd(p.back_count, 1ull)] = q;
         } else if (done) {
+          n_pred += cell.pred;
+          n_esc += cell.esc;
+          if (PRED == RPD_PRED_EXACT && p.exact_counters && cell.uncertain) {
+            atomicAdd(p.exact_counters, (unsigned long long)cell.uncertain);
+            if (cell.flips) atomicAdd(p.exact_counters + 1, (unsigned long long)cell.flips);
+          }
           int st = status;
           unsigned long long off = 0;
           if (emit) {
@@ -419,6 +428,7 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
         box.mid = make_float3(0.f, 0.f, 0.f);
         box.half = make_float3(INFINITY, INFINITY, INFINITY);
         box.R = INFINITY;
+        cell = {0u, 0u, 0u, 0u};
         status = kSuccess;
         out = kRun;
         cand = 0;
@@ -541,9 +551,14 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
           const int v = __ffs(und) - 1;
           und &= und - 1u;
           const uint32_t b = __float_as_uint(w.vx[v][lane].w);
-          if (slow_conflict<PRED>(w.pl[b & 15u][lane], w.pl[(b >> 4) & 15u][lane],
-                                  w.pl[(b >> 8) & 15u][lane], e, p.exact_counters, &n_esc))
-            some |= 1u << v;
+          const int x = slow_conflict<PRED>(w.pl[b & 15u][lane], w.pl[(b >> 4) & 15u][lane],
+                                            w.pl[(b >> 8) & 15u][lane], e);
+          if (x & kSignConflict) some |= 1u << v;
+          if (x & kSignEscalated) ++cell.esc;
+          if (PRED == RPD_PRED_EXACT) {
+            if (x & kSignUncertain) ++cell.uncertain;
+            if (x & kSignFlip) ++cell.flips;
+          }
           if (und == 0u) hit = some;
         }
         if (n_busy == 0) continue;
@@ -601,7 +616,7 @@ __global__ void __launch_bounds__(kTWarps * 32, kTBlocks) clip_threads_kernel(Cl
           if (s < -b) m |= 1u << v;
           else if (!(s > b)) un |= 1u << v;
         }
-        n_pred += (uint32_t)nv;
+        cell.pred += (uint32_t)nv;
         if (m | un) {
           last = u;
           e = f;
