@@ -116,7 +116,12 @@ __device__ float cone_distance(f3 p, float4 m1, float4 m2) {
     disc = (float)(((double)(D * D) - 4.0 * A * F) * (R1 * R1 - A) * R1 * R1);
   const float root = sqrtf(disc);
   float t = (-(A * D - R1 * R1 * D) - root) / (2.f * (A * A - A * R1 * R1));
-  t = fmaxf(0.f, fminf(t, 1.f));  // clamp to [0, 1] (saturation: a NaN becomes 0)
+  // clamp to [0, 1], a NaN to 0: where the larger sphere holds the smaller one
+  // the radicand is negative, and the distance, which only falls towards the
+  // larger one, is its own.  (fmaxf(0, fminf(t, 1)), the reference's clamp, gives
+  // the same here, as the compiler makes a saturation of it; by the functions'
+  // own rule for a NaN it would give 1, the smaller sphere.)
+  t = __saturatef(t);
   // t runs from the larger sphere m2 (t = 0) to m1 (t = 1): the reference's
   // lerp(a, b, t) is b + t (a - b) (include/cuda_helper_math.h:911-925)
   const float4 s = make_float4(m2.x + t * (m1.x - m2.x), m2.y + t * (m1.y - m2.y),
