@@ -84,13 +84,17 @@ typedef struct rpd_config {
   int knn_k;             /* list length for RPD_NEIGH_KNN, 1..128 */
   int clip_order;        /* rpd_clip_order (RPD_NEIGH_KNN only) */
   int compute_geometry;  /* 1: FP64 vertex coordinates and cell volumes */
-  int warps_per_block;   /* clip kernel block size in warps, 0 = default */
-  int blocks_per_sm;     /* persistent grid: blocks per SM, 0 = default */
+  int warps_per_block;   /* warp-per-cell clipper: block size in warps, 0 =
+                            default.  (It takes small passes, FP64 predicates,
+                            shortened lists, and the cells that outgrow the
+                            thread-per-cell clipper, which takes the rest and
+                            has no settings) */
+  int blocks_per_sm;     /* its persistent grid: blocks per SM, 0 = default */
   int certify;           /* 1 (RPD_NEIGH_KNN only): clip in ascending bisector
                             distance and stop at the security-radius
                             certificate; cells equal the plain path's up to
                             the order of their records (same topology) */
-  int clip_variant;      /* clip kernel register budget: 0 none (occupancy
+  int clip_variant;      /* its register budget: 0 none (occupancy
                             set by registers), 1 = 80 registers (6 blocks of
                             4 warps per SM), 2 = 64 registers (8 blocks) */
   int learned_k;         /* 1 (with certify): per-cell list lengths from the
@@ -163,7 +167,8 @@ typedef struct rpd_stats {
   int32_t knn_k;              /* neighbour list length used */
   float ms_total;             /* device time of rpd_compute, CUDA events */
   float ms_knn, ms_pairs, ms_clip, ms_compact;
-  float ms_clip_kernel;       /* the clip kernel alone (events around it) */
+  float ms_clip_kernel;       /* the first clipping pass alone (events around
+                                 its one or two kernels) */
   int32_t n_launches;         /* kernels launched by this rpd_compute */
   /* candidate search counters: [0] grid cells scanned, [1] cells kept after
    * the grown-cell planes, [2] tets enumerated, [3] tets inside the grown

@@ -1038,8 +1038,6 @@ rpd_status rpd_compute(rpd_ctx* c, rpd_stats* stats) {
         int bblocks = std::max(1, std::min((n_site + bw - 1) / bw, c->num_sms * box_blocks_per_sm(bw)));
         if (!second) CK(launch_site_box(bp, bblocks, bw, st), "site boxes");
         PairParams pp;
-        pp.vert3f = c->vert3f.ptr;
-        pp.tets = c->tets.ptr;
         pp.tet_base = 0;
         pp.site_base = 0;
         pp.tg = tg;

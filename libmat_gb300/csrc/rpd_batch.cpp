@@ -320,8 +320,6 @@ rpd_status front_end(rpd_batch* b) {
       const int bblocks = std::max(1, std::min((m.n_site + bw - 1) / bw, c->num_sms * box_blocks_per_sm(bw)));
       if (!second) BCK(launch_site_box(bp, bblocks, bw, ls), "site boxes");
       PairParams pp;
-      pp.vert3f = c->vert3f.ptr;
-      pp.tets = c->tets.ptr + tb;
       pp.tet_base = tb;
       pp.site_base = sb;
       pp.tg = tg;

@@ -43,20 +43,11 @@ namespace rpd {
 // ------------------------------------------------------------------------
 struct __align__(16) WarpCell {
   float4 pl[kMaxP];  // plane (a, b, c, d), inside: a x + b y + c z + d >= 0
-  union {
-    struct {
-      // of each vertex: its cofactors and the 3x3 permanents matching them
-      // (filter), or the four FP64 minors of its planes (FP64 predicates)
-      float4 K[kMaxT];
-      float4 M[kMaxT];
-      float rad[kMaxT]; // bound on each vertex's distance to the seed (certificate)
-    } f;
-    struct {
-      df n[kMaxP][3];   // plane normal, seed frame, double-float (geometry)
-      df d[kMaxP];      // plane offset, seed frame
-      float3 foot[kMaxP];  // foot of the volume origin on each plane
-    } g;
-  } u;
+  // of each vertex: its cofactors and the 3x3 permanents matching them
+  // (filter), or the four FP64 minors of its planes (FP64 predicates)
+  float4 K[kMaxT];
+  float4 M[kMaxT];
+  float rad[kMaxT];  // bound on each vertex's distance to the seed (certificate)
   int2 id2[kMaxP];
   uchar4 ver[kMaxT];
   uchar4 edge[kMaxE];
@@ -77,8 +68,8 @@ struct CellState {
 // rounds them.  (The FP64 pipe bounds this mode: 48k tets, 88M predicates, clip
 // stage 11.96 -> 5.17 ms.)
 __device__ __forceinline__ Minors load_minors(const WarpCell& c, int vi) {
-  const double2 a = reinterpret_cast<const double2*>(c.u.f.K)[vi];
-  const double2 b = reinterpret_cast<const double2*>(c.u.f.M)[vi];
+  const double2 a = reinterpret_cast<const double2*>(c.K)[vi];
+  const double2 b = reinterpret_cast<const double2*>(c.M)[vi];
   return {a.x, a.y, b.x, b.y};
 }
 // what the predicates (and with RAD the certificate) need of vertex vi
@@ -89,15 +80,15 @@ __device__ __forceinline__ void set_vertex(WarpCell& c, int vi, float4 p1, float
     float4 K, M;
     vertex_cofactors(p1, p2, p3, K, M);
     if (uses_filter(PRED)) {
-      c.u.f.K[vi] = K;
-      c.u.f.M[vi] = M;
+      c.K[vi] = K;
+      c.M[vi] = M;
     }
-    if (RAD) c.u.f.rad[vi] = vertex_radius(K, M, S);
+    if (RAD) c.rad[vi] = vertex_radius(K, M, S);
   }
   if (!uses_filter(PRED)) {
     const Minors m = det4x4_minors(p1, p2, p3);
-    reinterpret_cast<double2*>(c.u.f.K)[vi] = make_double2(m.m234, m.m134);
-    reinterpret_cast<double2*>(c.u.f.M)[vi] = make_double2(m.m124, m.m123);
+    reinterpret_cast<double2*>(c.K)[vi] = make_double2(m.m234, m.m134);
+    reinterpret_cast<double2*>(c.M)[vi] = make_double2(m.m124, m.m123);
   }
 }
 
@@ -111,12 +102,12 @@ __device__ __forceinline__ bool in_conflict(const WarpCell& c, int vi, float4 e,
   }
   ++pc.pred;
   if (uses_filter(PRED)) {
-    int s = filter_sign(c.u.f.K[vi], c.u.f.M[vi], e);
+    int s = filter_sign(c.K[vi], c.M[vi], e);
     if (s != 0) return s > 0;
     ++pc.esc;
     const uchar4 v = c.ver[vi];
     if (PRED == RPD_PRED_EXACT) {
-      const int x = exact_conflict(c.pl[v.x], c.pl[v.y], c.pl[v.z], e, c.u.f.M[vi]);
+      const int x = exact_conflict(c.pl[v.x], c.pl[v.y], c.pl[v.z], e, c.M[vi]);
       if (pc.exact && (x & kSignUncertain)) {
         atomicAdd(pc.exact, 1ull);
         if (x & kSignFlip) atomicAdd(pc.exact + 1, 1ull);
@@ -280,7 +271,7 @@ __device__ __forceinline__ uint64_t shfl64(uint64_t v, int src) {
 // the cell radius: the largest of the vertices' cached bounds
 __device__ __forceinline__ float cell_radius(const WarpCell& c, int nb_v, int lane) {
   float r = 0.f;
-  for (int v = lane; v < nb_v; v += 32) r = fmaxf(r, c.u.f.rad[v]);
+  for (int v = lane; v < nb_v; v += 32) r = fmaxf(r, c.rad[v]);
   for (int o = 16; o > 0; o >>= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
   return r;
 }
@@ -372,16 +363,16 @@ __device__ __noinline__ int partition_serial(WarpCell& c, int nb_v, uint32_t m0,
       const uchar4 tv = c.ver[i];
       c.ver[i] = c.ver[nb_v];
       c.ver[nb_v] = tv;
-      const float4 k = c.u.f.K[i];
-      c.u.f.K[i] = c.u.f.K[nb_v];
-      c.u.f.K[nb_v] = k;
-      const float4 mm = c.u.f.M[i];
-      c.u.f.M[i] = c.u.f.M[nb_v];
-      c.u.f.M[nb_v] = mm;
+      const float4 k = c.K[i];
+      c.K[i] = c.K[nb_v];
+      c.K[nb_v] = k;
+      const float4 mm = c.M[i];
+      c.M[i] = c.M[nb_v];
+      c.M[nb_v] = mm;
       if (RAD) {
-        const float r = c.u.f.rad[i];
-        c.u.f.rad[i] = c.u.f.rad[nb_v];
-        c.u.f.rad[nb_v] = r;
+        const float r = c.rad[i];
+        c.rad[i] = c.rad[nb_v];
+        c.rad[nb_v] = r;
       }
       const uint32_t wn = nb_v < 32 ? m0 : (nb_v < 64 ? m1 : m2);
       const uint32_t bit = 1u << (i & 31);
@@ -436,18 +427,18 @@ __device__ __forceinline__ void clip_full(WarpCell& c, CellState& s, const uint3
     if (move) {
       t = c.ver[src];
       if (v < n2) {
-        K = c.u.f.K[src];
-        M = c.u.f.M[src];
-        if (RAD) rd = c.u.f.rad[src];
+        K = c.K[src];
+        M = c.M[src];
+        if (RAD) rd = c.rad[src];
       }
     }
     __syncwarp();
     if (move) {
       c.ver[v] = t;
       if (v < n2) {
-        c.u.f.K[v] = K;
-        c.u.f.M[v] = M;
-        if (RAD) c.u.f.rad[v] = rd;
+        c.K[v] = K;
+        c.M[v] = M;
+        if (RAD) c.rad[v] = rd;
       }
     }
   } else {
@@ -658,9 +649,9 @@ __device__ void clip_list(WarpCell& c, CellState& s, const int32_t* list, int k,
         for (int v = lane; v < s.kept; v += 32) {
           const int src = c.perm[v];
           if (src != v) {
-            c.u.f.K[v] = c.u.f.K[src];
-            c.u.f.M[v] = c.u.f.M[src];
-            if (CERT) c.u.f.rad[v] = c.u.f.rad[src];
+            c.K[v] = c.K[src];
+            c.M[v] = c.M[src];
+            if (CERT) c.rad[v] = c.rad[src];
           }
         }
         __syncwarp();
@@ -674,9 +665,9 @@ __device__ void clip_list(WarpCell& c, CellState& s, const int32_t* list, int k,
           if (t.x == cur) {
             float4 K, M;
             vertex_cofactors(c.pl[t.x], c.pl[t.y], c.pl[t.z], K, M);
-            c.u.f.K[v] = K;
-            c.u.f.M[v] = M;
-            if (CERT) c.u.f.rad[v] = vertex_radius(K, M, cert.S);
+            c.K[v] = K;
+            c.M[v] = M;
+            if (CERT) c.rad[v] = vertex_radius(K, M, cert.S);
           }
         }
       }

@@ -175,13 +175,15 @@ inline int default_box_planes(int n_site, double w_max, const double* lo, const 
 size_t clip_smem_per_warp();
 int clip_blocks_per_sm(int pred_mode, int warps);
 int box_blocks_per_sm(int warps);
-// variant: 0 = no register cap (warps per block as given), 1 = at most 80
-// registers (6 blocks of 4 warps per SM), 2 = at most 64 (8 blocks of 4 warps)
-// one thread per cell, for the pairs of a first pass on whole base lists
-// (clip_threads_takes says which); what outgrows it lands in p.back_idx
+// one thread per cell, for the pairs of a first pass on whole base lists and
+// the exact-lists rounds' re-clips (clip_threads_takes says which); what
+// outgrows it lands in p.back_idx
 bool clip_threads_takes(const ClipParams& p, int pred_mode);
 cudaError_t launch_clip_threads(const ClipParams& p, int pred_mode, int certify, int num_sms,
                                 cudaStream_t st);
+// one warp per cell.  variant: 0 = no register cap (warps per block as given),
+// 1 = at most 80 registers (6 blocks of 4 warps per SM), 2 = at most 64 (8
+// blocks of 4 warps)
 cudaError_t launch_clip_cells(const ClipParams& p, int pred_mode, int certify, int variant,
                               int blocks, int warps, cudaStream_t st);
 int clip_blocks_per_sm_cert(int pred_mode, int certify, int warps, int variant);
@@ -268,8 +270,6 @@ cudaError_t launch_knn(const KnnArgs& a, cudaStream_t st);
 // candidate pairs: per site, tets whose centroid lies in the site's box and
 // that pass the reference rule; appends (tet, site) and counts per tet
 struct PairParams {
-  const float* vert3f;     // all vertices (tets hold global vertex ids)
-  const int4* tets;        // this mesh's tets
   int tet_base;            // index of this mesh's first tet among all tets
   int site_base;
   Grid tg;
