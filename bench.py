@@ -190,15 +190,31 @@ def clip_algorithmic_bytes(cfg, n_pairs, k, topo_bytes):
     return mesh + sites + 8 * k * ns + 8 * n_pairs + 32 * n_pairs + topo_bytes
 
 
-# DRAM traffic of one clip launch per candidate pair: ncu
-# dram__bytes_read.sum + dram__bytes_write.sum of clip_threads_kernel on the
-# 200k-tet ellipsoid (the same workload family, scaled by the launch's pairs:
-# its traffic grows with them), and smsp__issue_active of the same capture;
-# the capture and its command are summarised in
-# profiles/clip_threads_kernel_ellipsoid_200k.md
-CLIP_DRAM_BYTES_PER_PAIR = 304.1
-CLIP_ISSUE_ACTIVE = 0.499
-CLIP_THREADS_PER_INST = 14.18
+# The first clipping pass by lanes (FP32-filter or exact predicates, whole base
+# lists, at least CLIP_LANE_PAIRS pairs: kThreadsPairs of rpd_clip_thread.cu):
+# DRAM traffic per candidate pair of its two launches -- ncu
+# dram__bytes_read.sum + dram__bytes_write.sum of clip_threads_kernel and of
+# clip_cells_kernel on the cells that go back, 200k-tet ellipsoid (the same
+# workload family, scaled by the pass's pairs: its traffic grows with them) --
+# and smsp__issue_active and threads per instruction of the first, from the same
+# capture; its command is in profiles/clip_threads_kernel_ellipsoid_200k.md
+CLIP_LANE_PAIRS = 20000
+CLIP_DRAM_BYTES_PER_PAIR = 309.4
+CLIP_ISSUE_ACTIVE = 0.518
+CLIP_THREADS_PER_INST = 14.20
+
+
+def clip_pass(n_pairs, shortened):
+    """The kernels of a first clipping pass (ms_clip_kernel) and what was
+    captured of them: counters for the lanes' kernels, none for the others."""
+    if shortened or n_pairs < CLIP_LANE_PAIRS:
+        return {"kernel": "clip_cells_kernel", "traffic": None, "issue_active_frac": None,
+                "threads_per_inst": None}
+    return {"kernel": "clip_threads_kernel + clip_cells_kernel",
+            "traffic": CLIP_DRAM_BYTES_PER_PAIR * n_pairs,
+            # what bounds it instead of HBM: instruction issue and latency
+            # (of clip_threads_kernel)
+            "issue_active_frac": CLIP_ISSUE_ACTIVE, "threads_per_inst": CLIP_THREADS_PER_INST}
 
 
 def sample_tets(n_tet, n, seed):
@@ -557,7 +573,7 @@ def run_ours(args):
     xyz_bytes = 24 * int(fast_ph["nb_v"][ok].astype(np.int64).sum())
     alg = clip_algorithmic_bytes(cfg, st.n_pairs, st.knn_k, st.payload_bytes - xyz_bytes)
     achieved = alg / (st.ms_clip_kernel / 1000.0) / 1e9
-    traffic = CLIP_DRAM_BYTES_PER_PAIR * st.n_pairs
+    shortened = used_learned or bool(tuning and tuning["k_bucket"])
 
     cpu = parity = true_rpd = None
     if rank == 0 and not args.no_cpu:
@@ -632,15 +648,9 @@ def run_ours(args):
         "e2e": e2e,
         "topology": topology,
         "gpu_launches": int(st.n_launches) * args.steps,
-        "roofline": {"bound": "hbm", "kernel": "clip_threads_kernel", "achieved": achieved,
-                     "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
-                     "peak_source": peak_src,
-                     "algorithmic_bytes": alg,
-                     # what bounds it instead: instruction issue and
-                     # latency (ncu smsp__issue_active and threads per
-                     # executed instruction of the same kernel)
-                     "issue_active_frac": CLIP_ISSUE_ACTIVE,
-                     "threads_per_inst": CLIP_THREADS_PER_INST},
+        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                     "frac": achieved / peak, "peak_source": peak_src,
+                     "algorithmic_bytes": alg, **clip_pass(st.n_pairs, shortened)},
         "cpu_baseline": cpu,
         "clocks": clk.summary(),
     }
