@@ -264,10 +264,10 @@ rpd_status rpd_set_neighbors(struct rpd_ctx* ctx, const int32_t* nbr, int k,
 rpd_status rpd_set_site_k(struct rpd_ctx* ctx, const int32_t* k_per_site, int on_device);
 
 /* Autotuner: times rpd_compute on the context's current inputs for each
- * candidate launch configuration of the clip kernel -- block size 2, 4 or 8
- * warps, register budgets for 16, 24 or 32 resident warps per SM (the
- * shared-memory budget per SM follows: 5.7 KB per warp) -- and, with
- * config.certify, first-pass list lengths of 16, 32 or all neighbours
+ * candidate launch configuration of the warp-per-cell clipper (the
+ * thread-per-cell one has none) -- block size 2, 4 or 8 warps, register
+ * budgets for 16, 24 or 32 resident warps per SM (the shared-memory budget
+ * per SM follows: 5.7 KB per warp) -- and, with config.certify, first-pass list lengths of 16, 32 or all neighbours
  * (k-bucket; cells not certified by their bucket are clipped again whole)
  * and, once a k-predictor is trained or loaded, its per-cell lengths.
  * Keeps the fastest in the context (the cells are the same for every
